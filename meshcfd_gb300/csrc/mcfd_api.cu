@@ -668,6 +668,9 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   size_t o_saved = A.take(bytes_d(4 * C));
   size_t o_partials = A.take(bytes_d(4 * partial_blocks));
   size_t o_bc_ext = A.take(bytes_d(4 * NB)), o_bc_ext_dt = A.take(bytes_d(4 * NB)), o_bc_terms = A.take(bytes_d(NB));
+  const size_t par_cells = NE ? (size_t)C : 0;
+  size_t o_par_fit = A.take(bytes_d(kParFit * par_cells)), o_par_rec = A.take(bytes_d(6 * NE)),
+         o_par_full = A.take(bytes_i(par_cells));
 
   mcfd_geom* h = new mcfd_geom();
   cudaError_t err = cudaMalloc(&h->arena, A.size);
@@ -677,7 +680,7 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   }
   h->arena_bytes = A.size;
   char* base = static_cast<char*>(h->arena);
-  std::vector<char> host(A.size, 0);
+  std::vector<char> host(o_P, 0);  // the geometry part; the workspace has no host image
   auto put = [&](size_t off, const void* src, size_t bytes) {
     if (bytes) std::memcpy(host.data() + off, src, bytes);
   };
@@ -780,6 +783,9 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   g.par_ptr = AT(const int*, o_par_ptr);
   g.par_nb = AT(const int*, o_par_nb);
   g.par_d = AT(const double2*, o_par_d);
+  g.par_fit = AT(const double*, o_par_fit);
+  g.par_rec = AT(const double*, o_par_rec);
+  g.par_full = AT(const int*, o_par_full);
   g.n_bc_patches = (int)NBP;
   g.bc_ptr = AT(const int*, o_bc_ptr);
   g.bc_kind = AT(const int*, o_bc_kind);
@@ -880,6 +886,16 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
       t.boundary_owner.push_back((int)d->owners[f]);
       t.boundary_normal.push_back(make_double2(d->face_normals[2 * f], d->face_normals[2 * f + 1]));
       t.boundary_len.push_back(d->face_lengths[f]);
+    }
+  }
+  if (NE > 0) {  // the parabolic fit's mesh-only part
+    err = launch_parabolic_plan(g, reinterpret_cast<double*>(base + o_par_fit),
+                                reinterpret_cast<double*>(base + o_par_rec),
+                                reinterpret_cast<int*>(base + o_par_full), nullptr);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
+    if (err != cudaSuccess) {
+      mcfd_geom_destroy(h);
+      return MCFD_E_CUDA;
     }
   }
   *out = h;

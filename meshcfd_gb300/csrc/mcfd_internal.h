@@ -55,6 +55,10 @@ struct DevGeom {
   const int* par_ptr;
   const int* par_nb;
   const double2* par_d;
+  // the fit's mesh-only part (launch_parabolic_plan, at creation)
+  const double* par_fit;  // [kParFit][C] LU, reciprocals, scale
+  const double* par_rec;  // [n_parabolic][6] weight x basis in pivoted row order, neighbour
+  const int* par_full;    // [C] 1 where the normal matrix has full rank
   // flux faces
   const int* ff_lslot;  // recon slot of the interior-side state
   const int* ff_rslot;  // recon slot of the other side (interior/periodic), else -1
@@ -222,6 +226,8 @@ cudaError_t launch_case_time_steps(int n_cells, int n_cases, const int* offsets,
                                    double* dt_cells, cudaStream_t s);
 // MUSCL parabolic and the reference's reconstruction fields (mcfd_parabolic.cu;
 // exact arithmetic in every mode)
+constexpr int kParFit = 34;  // doubles per cell of DevGeom::par_fit
+cudaError_t launch_parabolic_plan(const DevGeom& g, double* fit, double* rec, int* full, cudaStream_t s);
 cudaError_t launch_reconstruct_parabolic(const DevGeom& g, const mcfd_config& cfg, const double* P, double* recon,
                                          cudaStream_t s);
 cudaError_t launch_reconstruction_fields(const DevGeom& g, const mcfd_config& cfg, const double* P, double* grad,

@@ -1,18 +1,24 @@
 // MUSCL-parabolic reconstruction and the reference's reconstruction fields.
 //
-// _parabolic_reconstruction (solver.py:2322-2415), per cell (one thread):
+// _parabolic_reconstruction (solver.py:2322-2415).  Per cell, from the mesh
+// alone (k_parabolic_plan, once per geometry, one thread per cell):
 //   * the stencil scale max(|dx|, |dy|) over the cell's two-ring entries;
-//   * the weighted normal equations M (5x5) and right-hand sides B (5x4),
-//     accumulated over the cell's entries in the reference's entry order
-//     (np.add.at is sequential), weights 1 / max(|r/scale|^2, 1e-300);
+//   * the weighted normal equations M (5x5), accumulated over the cell's
+//     entries in the reference's entry order (np.add.at is sequential),
+//     weights 1 / max(|r/scale|^2, 1e-300);
 //   * the rank gate np.linalg.matrix_rank(M) == 5: an LU with partial
 //     pivoting gives the Frobenius condition number kappa_F = |M| |M^-1|;
 //     below 1e12 the matrix is certainly of full rank (s_min / s_max >=
 //     1 / kappa_F, far above the 5 eps threshold), otherwise one-sided
 //     Jacobi singular values (Hestenes' method) and the rank rule decide;
-//   * the solve by the same LU (row interchange to the first largest
-//     |a_ik|, unit lower factor, right-looking); np.linalg.solve's LAPACK
-//     gesv agrees to rounding (a few 1e-15 relative), not bit for bit;
+//   * that LU's factors (row interchange to the first largest |a_ik|, unit
+//     lower factor, right-looking), and per entry the five products weight x
+//     basis in the order of the interchanged rows, so that the right-hand
+//     side accumulates in its pivoted order.
+// Per state (k_reconstruct_parabolic, one thread per cell and variable):
+//   * the variable's right-hand side, accumulated over the entries in order;
+//   * the solve by the stored LU; np.linalg.solve's LAPACK gesv agrees to
+//     rounding (a few 1e-15 relative), not bit for bit;
 //   * the limiter on the quadratic increment with two-ring extrema, or, for
 //     cells that fail the gate, the linear gradient and limiter of
 //     _limited_gradients (identical to the linear kernels, entry order kept).
@@ -222,152 +228,307 @@ __device__ __forceinline__ void linear_cell(const DevGeom& g, const double* __re
   }
 }
 
-template <int LIMITER, bool PARABOLIC, bool FIELDS>
-__global__ void __launch_bounds__(kBlock) k_reconstruct_full(DevGeom g, const double* __restrict__ P,
-                                                             double* __restrict__ recon, double* __restrict__ grad_out,
-                                                             double* __restrict__ curv_out,
-                                                             double* __restrict__ fac_out) {
+// The linear fields of the reference (mcfd_reconstruction), one thread per cell.
+template <int LIMITER>
+__global__ void __launch_bounds__(kBlock) k_linear_fields(DevGeom g, const double* __restrict__ P,
+                                                          double* __restrict__ grad_out,
+                                                          double* __restrict__ fac_out) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.n_cells) return;
   const St4 p = ld4(P + 4 * (size_t)c);
   const double pv[4] = {p.a, p.b, p.c, p.d};
-  double gx[4], gy[4], kxx[4] = {0, 0, 0, 0}, kxy[4] = {0, 0, 0, 0}, kyy[4] = {0, 0, 0, 0}, phi[4];
-  bool full = false;
-  if (PARABOLIC && g.n_parabolic > 0) {
-    const int e0 = g.par_ptr[c], e1 = g.par_ptr[c + 1];
-    double scale = 0.0;
-    for (int e = e0; e < e1; ++e) {
-      const double2 d = g.par_d[e];
-      const double a = fabs(d.x), b = fabs(d.y);
-      const double m = a >= b ? a : b;
-      if (m > scale) scale = m;
-    }
-    if (!(scale >= 1e-300)) scale = 1e-300;
-    double M[5][5], B[5][4], lo[4], hi[4];
+  double gx[4], gy[4], phi[4];
+  linear_cell<LIMITER>(g, P, c, pv, gx, gy, phi);
 #pragma unroll
-    for (int i = 0; i < 5; ++i) {
+  for (int v = 0; v < 4; ++v) {
+    grad_out[8 * (size_t)c + 2 * v] = gx[v];
+    grad_out[8 * (size_t)c + 2 * v + 1] = gy[v];
+    fac_out[4 * (size_t)c + v] = phi[v];
+  }
+}
+
+// Everything of a cell's fit that depends on the mesh alone.  The normal
+// matrix, its LU, the inverse of the rank gate and the weights were some 85 %
+// of the former one-kernel reconstruction's operations; they are the same for
+// every state, so they are computed once, when the geometry is created.
+// fit: [kParFit][C], the LU row by row (25), the fixed-point reciprocals of
+// its diagonal (5), the scale, its square and their reciprocals (4); rec:
+// [entries][6], the weight x basis products in pivoted row order and the
+// neighbour's index; full: whether the cell passes the rank gate.
+__global__ void __launch_bounds__(kBlock) k_parabolic_plan(DevGeom g, double* __restrict__ fit,
+                                                           double* __restrict__ rec, int* __restrict__ full_out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= g.n_cells) return;
+  const int e0 = g.par_ptr[c], e1 = g.par_ptr[c + 1];
+  double scale = 0.0;
+  for (int e = e0; e < e1; ++e) {
+    const double2 d = g.par_d[e];
+    const double a = fabs(d.x), b = fabs(d.y);
+    const double m = a >= b ? a : b;
+    if (m > scale) scale = m;
+  }
+  if (!(scale >= 1e-300)) scale = 1e-300;
+  auto products = [&](int e, double (&dd)[5], double (&wd)[5]) {
+    const double2 d = g.par_d[e];
+    const double nx = div_rn(d.x, scale), ny = div_rn(d.y, scale);
+    dd[0] = nx;
+    dd[1] = ny;
+    dd[2] = 0.5 * (nx * nx);
+    dd[3] = nx * ny;
+    dd[4] = 0.5 * (ny * ny);
+    const double r2 = nx * nx + ny * ny;
+    const double w = div_rn(1.0, r2 >= 1e-300 ? r2 : 1e-300);
 #pragma unroll
-      for (int j = 0; j < 5; ++j) M[i][j] = 0.0;
+    for (int i = 0; i < 5; ++i) wd[i] = w * dd[i];
+  };
+  double M[5][5];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) B[i][v] = 0.0;
-    }
+  for (int i = 0; i < 5; ++i)
 #pragma unroll
-    for (int v = 0; v < 4; ++v) lo[v] = hi[v] = pv[v];
-    for (int e = e0; e < e1; ++e) {
-      const double2 d = g.par_d[e];
-      const double nx = div_rn(d.x, scale), ny = div_rn(d.y, scale);
-      const double dd[5] = {nx, ny, 0.5 * (nx * nx), nx * ny, 0.5 * (ny * ny)};
-      const double r2 = nx * nx + ny * ny;
-      const double w = div_rn(1.0, r2 >= 1e-300 ? r2 : 1e-300);
-      const St4 q = ld4(P + 4 * (size_t)g.par_nb[e]);
-      const double qv[4] = {q.a, q.b, q.c, q.d};
-      double diff[4];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        diff[v] = qv[v] - pv[v];
-        if (icmp::lt(qv[v], lo[v])) lo[v] = qv[v];
-        if (icmp::lt(hi[v], qv[v])) hi[v] = qv[v];
-      }
-#pragma unroll
-      for (int i = 0; i < 5; ++i) {
-        const double wi = w * dd[i];
-#pragma unroll
-        for (int j = 0; j < 5; ++j) M[i][j] += wi * dd[j];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) B[i][v] += wi * diff[v];
-      }
-    }
-    double LU[5][5];
+    for (int j = 0; j < 5; ++j) M[i][j] = 0.0;
+  for (int e = e0; e < e1; ++e) {
+    double dd[5], wd[5];
+    products(e, dd, wd);
 #pragma unroll
     for (int i = 0; i < 5; ++i)
 #pragma unroll
-      for (int j = 0; j < 5; ++j) LU[i][j] = M[i][j];
-    int piv[5] = {0, 1, 2, 3, 4};
-    const bool ok = lu5(LU, piv);
-    full = full_rank5(M, LU, piv, ok);
-    if (full) {
-      lu5_solve<4>(LU, piv, B);
-      const double sc = scale, sc2 = scale * scale;
+      for (int j = 0; j < 5; ++j) M[i][j] += wd[i] * dd[j];
+  }
+  double LU[5][5];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        gx[v] = div_rn(B[0][v], sc);
-        gy[v] = div_rn(B[1][v], sc);
-        kxx[v] = div_rn(B[2][v], sc2);
-        kxy[v] = div_rn(B[3][v], sc2);
-        kyy[v] = div_rn(B[4][v], sc2);
-        phi[v] = 1.0;
-      }
-      const int s0 = g.lim_ptr[c], s1 = g.lim_ptr[c + 1];
+  for (int i = 0; i < 5; ++i)
+#pragma unroll
+    for (int j = 0; j < 5; ++j) LU[i][j] = M[i][j];
+  int piv[5] = {0, 1, 2, 3, 4};
+  const bool ok = lu5(LU, piv);
+  full_out[c] = full_rank5(M, LU, piv, ok) ? 1 : 0;
+  const size_t C = g.n_cells;
+#pragma unroll
+  for (int i = 0; i < 5; ++i) {
+#pragma unroll
+    for (int j = 0; j < 5; ++j) fit[(5 * i + j) * C + c] = LU[i][j];
+    fit[(25 + i) * C + c] = __longlong_as_double((long long)recip_fixed(LU[i][i]));
+  }
+  const double sc2 = scale * scale;
+  fit[30 * C + c] = scale;
+  fit[31 * C + c] = sc2;
+  fit[32 * C + c] = __longlong_as_double((long long)recip_fixed(scale));
+  fit[33 * C + c] = __longlong_as_double((long long)recip_fixed(sc2));
+  // the products' row of each pivoted row, by the solve's own interchanges
+  // (a failed LU leaves no solve: any order)
+  for (int e = e0; e < e1; ++e) {
+    double dd[5], wd[5], b[5][1];
+    products(e, dd, wd);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) b[i][0] = wd[i];
+    swap_rows<0, 1>(b, piv[0]);
+    swap_rows<1, 1>(b, piv[1]);
+    swap_rows<2, 1>(b, piv[2]);
+    swap_rows<3, 1>(b, piv[3]);
+    double2* dst = reinterpret_cast<double2*>(rec + 6 * (size_t)e);
+    dst[0] = make_double2(b[0][0], b[1][0]);
+    dst[1] = make_double2(b[2][0], b[3][0]);
+    dst[2] = make_double2(b[4][0], __longlong_as_double((long long)g.par_nb[e]));
+  }
+}
+
+// Products of the right-hand side that run on the integer pipe (mul_rn, the
+// same IEEE product): the first MCFD_PAR_INT_MUL of an entry's five.  RK3 step
+// of the 181 x 181 vortex with 0 / 1 / 2 / 3 / 5 of them: 600 / 561 / 557 /
+// 558 / 544 us; and with 8 / 10 / 11 / 12 resident 128-thread blocks: 541 /
+// 545 / 532 / 533 us.
+#ifndef MCFD_PAR_INT_MUL
+#define MCFD_PAR_INT_MUL 5
+#endif
+#ifndef MCFD_PAR_MIN_BLOCKS
+#define MCFD_PAR_MIN_BLOCKS 11
+#endif
+template <int I>
+__device__ __forceinline__ double rhs_mul(double a, double b) {
+  if constexpr (I < MCFD_PAR_INT_MUL) return mul_rn(a, b);
+  else return a * b;
+}
+
+// Limiter factor and face states (or fields) of one variable for NS limiter
+// entries (NS = 0: any count, recomputing the increments).  The two sums of
+// the increment associate differently, as the reference's limiter and its
+// _reconstruct do; they share their products.
+template <int LIMITER, int NS>
+__device__ __forceinline__ double parabolic_faces(const DevGeom& g, double* __restrict__ recon, int v, double pv,
+                                                  int s0, int s1, double gx, double gy, double kxx, double kxy,
+                                                  double kyy, double lo, double hi) {
+  const double tol = limiter_tolerance(pv);
+  const double hxx = 0.5 * kxx, hyy = 0.5 * kyy;
+  double phi = 1.0;
+  if constexpr (NS > 0) {
+    double out[NS];
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const double2 d = g.lim_d[s0 + k];
+      const double t1 = gx * d.x + gy * d.y, txx = hxx * (d.x * d.x), txy = kxy * (d.x * d.y),
+                   tyy = hyy * (d.y * d.y);
+      out[k] = t1 + ((txx + txy) + tyy);
+      const double f = limiter_face_factor<LIMITER>(pv, ((t1 + txx) + txy) + tyy, lo, hi, tol);
+      if (icmp::lt_nonneg(f, phi)) phi = f;
+    }
+    if (recon) {
+#pragma unroll
+      for (int k = 0; k < NS; ++k) recon[4 * (size_t)g.lim_slot[s0 + k] + v] = pv + phi * out[k];
+    }
+  } else {
+    for (int s = s0; s < s1; ++s) {
+      const double2 d = g.lim_d[s];
+      const double inc = gx * d.x + gy * d.y + hxx * (d.x * d.x) + kxy * (d.x * d.y) + hyy * (d.y * d.y);
+      const double f = limiter_face_factor<LIMITER>(pv, inc, lo, hi, tol);
+      if (icmp::lt_nonneg(f, phi)) phi = f;
+    }
+    if (recon) {
       for (int s = s0; s < s1; ++s) {
         const double2 d = g.lim_d[s];
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          const double inc = gx[v] * d.x + gy[v] * d.y + 0.5 * kxx[v] * (d.x * d.x) + kxy[v] * (d.x * d.y) +
-                             0.5 * kyy[v] * (d.y * d.y);
-          const double f = limiter_face_factor<LIMITER>(pv[v], inc, lo[v], hi[v], limiter_tolerance(pv[v]));
-          if (f < phi[v]) phi[v] = f;
-        }
+        double inc = gx * d.x + gy * d.y;
+        inc += hxx * (d.x * d.x) + kxy * (d.x * d.y) + hyy * (d.y * d.y);
+        recon[4 * (size_t)g.lim_slot[s] + v] = pv + phi * inc;
       }
     }
   }
-  if (!full) linear_cell<LIMITER>(g, P, c, pv, gx, gy, phi);
-  if (FIELDS) {
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      grad_out[8 * (size_t)c + 2 * v] = gx[v];
-      grad_out[8 * (size_t)c + 2 * v + 1] = gy[v];
-      fac_out[4 * (size_t)c + v] = phi[v];
-      if (curv_out) {
-        curv_out[12 * (size_t)c + 3 * v] = kxx[v];
-        curv_out[12 * (size_t)c + 3 * v + 1] = kxy[v];
-        curv_out[12 * (size_t)c + 3 * v + 2] = kyy[v];
-      }
-    }
-    return;
-  }
+  return phi;
+}
+
+// One thread per (cell, variable): the variables of a cell are independent
+// given the plan, and four short threads leave room for the warps that hide
+// the 64-cycle FP64 latency (the former thread per cell held 246 registers).
+// Bound by the FP64 pipe (63 % busy at 49,141 cells, where the grid is a
+// little over one wave).  RK3 step of the 181 x 181 mixed vortex: 465 us per
+// reconstruction with the plan recomputed in it, 142 us now; the step 1,372
+// against 532 us.
+template <int LIMITER, bool FIELDS>
+__global__ void __launch_bounds__(kBlock, MCFD_PAR_MIN_BLOCKS) k_reconstruct_parabolic(DevGeom g, const double* __restrict__ P,
+                                                                  double* __restrict__ recon,
+                                                                  double* __restrict__ grad_out,
+                                                                  double* __restrict__ curv_out,
+                                                                  double* __restrict__ fac_out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = t >> 2, v = t & 3;
+  if (c >= g.n_cells) return;
+  const double pv = P[4 * (size_t)c + v];
   const int s0 = g.lim_ptr[c], s1 = g.lim_ptr[c + 1];
-  for (int s = s0; s < s1; ++s) {
-    const double2 d = g.lim_d[s];
-    double out[4];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      double inc = gx[v] * d.x + gy[v] * d.y;
-      if (PARABOLIC) inc += 0.5 * kxx[v] * (d.x * d.x) + kxy[v] * (d.x * d.y) + 0.5 * kyy[v] * (d.y * d.y);
-      out[v] = pv[v] + phi[v] * inc;
+  double gx = 0.0, gy = 0.0, kxx = 0.0, kxy = 0.0, kyy = 0.0, phi, lo = pv, hi = pv;
+  bool limited = true;
+  if (g.n_parabolic > 0 && g.par_full[c]) {
+    double b[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    for (int e = g.par_ptr[c], e1 = g.par_ptr[c + 1]; e < e1; ++e) {
+      const double2* r = reinterpret_cast<const double2*>(g.par_rec + 6 * (size_t)e);
+      const double2 r0 = r[0], r1 = r[1], r2 = r[2];
+      const double q = P[4 * (size_t)(int)__double_as_longlong(r2.y) + v];
+      const double diff = q - pv;
+      if (icmp::lt(q, lo)) lo = q;
+      if (icmp::lt(hi, q)) hi = q;
+      b[0] += rhs_mul<0>(r0.x, diff);
+      b[1] += rhs_mul<1>(r0.y, diff);
+      b[2] += rhs_mul<2>(r1.x, diff);
+      b[3] += rhs_mul<3>(r1.y, diff);
+      b[4] += rhs_mul<4>(r2.x, diff);
     }
-    st4(recon + 4 * (size_t)g.lim_slot[s], St4{out[0], out[1], out[2], out[3]});
+    const size_t C = g.n_cells;
+    const double* f = g.par_fit + c;
+#pragma unroll
+    for (int i = 1; i < 5; ++i)
+#pragma unroll
+      for (int j = 0; j < i; ++j) b[i] = b[i] - f[(5 * i + j) * C] * b[j];
+#pragma unroll
+    for (int i = 4; i >= 0; --i) {
+#pragma unroll
+      for (int j = i + 1; j < 5; ++j) b[i] = b[i] - f[(5 * i + j) * C] * b[j];
+      b[i] = div_rn_recip(b[i], f[(5 * i + i) * C], (unsigned long long)__double_as_longlong(f[(25 + i) * C]));
+    }
+    const double sc = f[30 * C], sc2 = f[31 * C];
+    const unsigned long long x1 = (unsigned long long)__double_as_longlong(f[32 * C]),
+                             x2 = (unsigned long long)__double_as_longlong(f[33 * C]);
+    gx = div_rn_recip(b[0], sc, x1);
+    gy = div_rn_recip(b[1], sc, x1);
+    kxx = div_rn_recip(b[2], sc2, x2);
+    kxy = div_rn_recip(b[3], sc2, x2);
+    kyy = div_rn_recip(b[4], sc2, x2);
+  } else {  // linear gradient and limiter (linear_cell, one variable): zero curvature
+    for (int e = g.grad_ptr[c], e1 = g.grad_ptr[c + 1]; e < e1; ++e) {
+      const double q = P[4 * (size_t)g.grad_nb[e] + v];
+      const double d = q - pv;
+      gx = gx + g.grad_cx[e] * d;
+      gy = gy + g.grad_cy[e] * d;
+      if (icmp::lt(q, lo)) lo = q;
+      if (icmp::lt(hi, q)) hi = q;
+    }
+    limited = g.n_gradient > 0;
+  }
+  double* out = FIELDS ? nullptr : recon;
+  if (!limited) {  // no gradient entries at all: zeros and ones (solver.py:2298-2302)
+    phi = 1.0;
+    if (!FIELDS)
+      for (int s = s0; s < s1; ++s) recon[4 * (size_t)g.lim_slot[s] + v] = pv + 0.0;
+  } else if (s1 - s0 == 3) {
+    phi = parabolic_faces<LIMITER, 3>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
+  } else if (s1 - s0 == 4) {
+    phi = parabolic_faces<LIMITER, 4>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
+  } else {
+    phi = parabolic_faces<LIMITER, 0>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
+  }
+  if (FIELDS) {
+    grad_out[8 * (size_t)c + 2 * v] = gx;
+    grad_out[8 * (size_t)c + 2 * v + 1] = gy;
+    fac_out[4 * (size_t)c + v] = phi;
+    if (curv_out) {
+      curv_out[12 * (size_t)c + 3 * v] = kxx;
+      curv_out[12 * (size_t)c + 3 * v + 1] = kxy;
+      curv_out[12 * (size_t)c + 3 * v + 2] = kyy;
+    }
   }
 }
 
 inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
 
-template <bool PARABOLIC, bool FIELDS>
-cudaError_t launch_full(const DevGeom& g, int limiter, const double* P, double* recon, double* grad, double* curv,
-                        double* fac, cudaStream_t s) {
+template <bool FIELDS>
+cudaError_t launch_parabolic(const DevGeom& g, int limiter, const double* P, double* recon, double* grad, double* curv,
+                             double* fac, cudaStream_t s) {
   if (g.n_cells == 0) return cudaSuccess;
-  const int b = blocks_for(g.n_cells);
+  const int b = (int)((4LL * g.n_cells + kBlock - 1) / kBlock);
   count_launch();
   switch (limiter) {
-    case 0: k_reconstruct_full<0, PARABOLIC, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
-    case 1: k_reconstruct_full<1, PARABOLIC, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
-    case 2: k_reconstruct_full<2, PARABOLIC, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
-    default: k_reconstruct_full<3, PARABOLIC, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
+    case 0: k_reconstruct_parabolic<0, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
+    case 1: k_reconstruct_parabolic<1, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
+    case 2: k_reconstruct_parabolic<2, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
+    default: k_reconstruct_parabolic<3, FIELDS><<<b, kBlock, 0, s>>>(g, P, recon, grad, curv, fac); break;
   }
   return cudaGetLastError();
 }
 
 }  // namespace
 
+cudaError_t launch_parabolic_plan(const DevGeom& g, double* fit, double* rec, int* full, cudaStream_t s) {
+  if (g.n_cells == 0 || g.n_parabolic == 0) return cudaSuccess;
+  count_launch();
+  k_parabolic_plan<<<blocks_for(g.n_cells), kBlock, 0, s>>>(g, fit, rec, full);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_reconstruct_parabolic(const DevGeom& g, const mcfd_config& cfg, const double* P, double* recon,
                                          cudaStream_t s) {
-  return launch_full<true, false>(g, cfg.limiter, P, recon, nullptr, nullptr, nullptr, s);
+  return launch_parabolic<false>(g, cfg.limiter, P, recon, nullptr, nullptr, nullptr, s);
 }
 
 cudaError_t launch_reconstruction_fields(const DevGeom& g, const mcfd_config& cfg, const double* P, double* grad,
                                          double* curv, double* fac, cudaStream_t s) {
   if (cfg.reconstruction == MCFD_RECON_MUSCL_PARABOLIC)
-    return launch_full<true, true>(g, cfg.limiter, P, nullptr, grad, curv, fac, s);
-  return launch_full<false, true>(g, cfg.limiter, P, nullptr, grad, curv, fac, s);
+    return launch_parabolic<true>(g, cfg.limiter, P, nullptr, grad, curv, fac, s);
+  if (g.n_cells == 0) return cudaSuccess;
+  const int b = blocks_for(g.n_cells);
+  count_launch();
+  switch (cfg.limiter) {
+    case 0: k_linear_fields<0><<<b, kBlock, 0, s>>>(g, P, grad, fac); break;
+    case 1: k_linear_fields<1><<<b, kBlock, 0, s>>>(g, P, grad, fac); break;
+    case 2: k_linear_fields<2><<<b, kBlock, 0, s>>>(g, P, grad, fac); break;
+    default: k_linear_fields<3><<<b, kBlock, 0, s>>>(g, P, grad, fac); break;
+  }
+  return cudaGetLastError();
 }
 
 }  // namespace mcfd
