@@ -86,8 +86,8 @@ __device__ __forceinline__ Dual<N> fabs(const Dual<N>& a) {
 template <int N>
 __device__ __forceinline__ Dual<N> pow(const Dual<N>& a, double e) {
   Dual<N> r;
-  r.v = ::pow(a.v, e);
-  const double g = e * ::pow(a.v, e - 1.0);
+  r.v = pow_rn(a.v, e);
+  const double g = e * pow_rn(a.v, e - 1.0);
 #pragma unroll
   for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * g;
   return r;

@@ -101,7 +101,7 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
       }
       const double m = 0.5 * (low + high);
       const double t = div_rn(tt, 1.0 + 0.5 * (gamma - 1.0) * (m * m));
-      const double p = pt * pow(div_rn(t, tt), div_rn(gamma, gamma - 1.0));
+      const double p = pt * pow_rn(div_rn(t, tt), div_rn(gamma, gamma - 1.0));
       const double rho = div_rn(p, R * t);
       const double speed = m * sqrt_rn(gamma * R * t);
       out = St4{rho, speed * dx, speed * dy, p};

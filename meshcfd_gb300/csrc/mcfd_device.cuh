@@ -10,6 +10,7 @@
 
 #include "../../include/meshcfd_gb300.h"
 #include "mcfd_arith.cuh"
+#include "mcfd_pow.cuh"
 
 namespace mcfd {
 
@@ -307,9 +308,9 @@ __device__ __forceinline__ int far_field_state(const St4& in, const St4& far, do
     return MCFD_S_FARFIELD_SOUND;
   }
   const St4& src = icmp::ge0(vb) ? in : far;
-  double entropy = div_rn(src.d, pow(src.a, gamma));
-  double rho = pow(div_rn(cb * cb, gamma * entropy), div_rn(1.0, gamma - 1.0));
-  double p = entropy * pow(rho, gamma);
+  double entropy = div_rn(src.d, pow_rn(src.a, gamma));
+  double rho = pow_rn(div_rn(cb * cb, gamma * entropy), div_rn(1.0, gamma - 1.0));
+  double p = entropy * pow_rn(rho, gamma);
   double tx = -ny, ty = nx;
   double vt = src.b * tx + src.c * ty;
   St4 s{rho, vb * nx + vt * tx, vb * ny + vt * ty, p};

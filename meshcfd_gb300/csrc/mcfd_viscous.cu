@@ -49,7 +49,7 @@ struct Visc {
 // _dynamic_viscosity; *bad set when Sutherland's law gives an invalid value
 __device__ __forceinline__ double viscosity(const Visc& v, double T, bool* bad) {
   if (v.model == MCFD_VISC_CONSTANT) return v.mu0;
-  double mu = v.suth_mu * pow(div_rn(T, v.suth_t), 1.5);
+  double mu = v.suth_mu * pow_rn(div_rn(T, v.suth_t), 1.5);
   mu *= div_rn(v.suth_t + v.suth_s, T + v.suth_s);
   if (!isfinite(mu) || !(mu > 0.0)) *bad = true;
   return mu;
