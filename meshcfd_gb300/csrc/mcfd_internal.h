@@ -198,14 +198,16 @@ MCFD_DECLARE_LAUNCHERS(fast)
 MCFD_DECLARE_LAUNCHERS(fma)
 #undef MCFD_DECLARE_LAUNCHERS
 
-// Launch shape of a face segment: 256-thread blocks when the segment fills
-// the 152 SMs, otherwise warp-multiple blocks spread over all SMs (a boundary
-// segment of a few thousand faces would sit on a handful of SMs).
+// Launch shape of a pass over n items: the FP64 pipe that bounds these kernels
+// is one per SM, so a launch takes as long as its fullest SM.  Small blocks
+// deal the items out evenly while there are few per SM, larger ones keep
+// the block count down once the remainder no longer matters (RK3 steps of
+// 41,000, 135,000 and 240,000 faces 137 -> 127, 228 -> 217 and 480 -> 451 us
+// against 256-thread blocks wherever they fill the SMs).
 inline int seg_threads(int n) {
-  if (n >= 152 * 256) return 256;
-  int t = (n + 151) / 152;
-  t = ((t + 31) / 32) * 32;
-  return t < 32 ? 32 : (t > 256 ? 256 : t);
+  if (n < 152 * 32 * 8) return 32;
+  if (n < 152 * 64 * 16) return 64;
+  return n < 152 * 128 * 16 ? 128 : 256;
 }
 inline int seg_blocks(int n) { return (n + seg_threads(n) - 1) / seg_threads(n); }
 // flux launch shape with the autotuned threads / faces per thread, if any

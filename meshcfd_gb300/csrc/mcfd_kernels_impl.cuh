@@ -35,6 +35,10 @@
 #define MCFD_FLUX_INT_MUL 4
 #endif
 
+#if MCFD_FAST == 0
+#define MCFD_LIBRARY_POW  // far_pow (mcfd_device.cuh)
+#endif
+
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -538,6 +542,38 @@ __global__ void __launch_bounds__(kBlock) k_flux(DevGeom g, const double* __rest
     flux_face<FLUX, SEG, FIRST_ORDER, KERNEL_HLLC>(g, P, recon, flux, gamma, inv_gm1, f, begin);
 }
 
+// Every segment in one launch, for meshes of at most kMergedFluxFaces faces:
+// a block belongs to one segment (warp-uniform code), the long chains first
+// (far field, then the other boundaries), the interior last.  A launch per
+// segment there costs more than it computes: the boundary segments go to a
+// side stream between a fork and a join, some 10 us a stage.  Bound by the
+// latency of the far-field chain.
+template <int FLUX, bool FIRST_ORDER, bool KERNEL_HLLC>
+__global__ void __launch_bounds__(kBlock) k_flux_merged(DevGeom g, const double* __restrict__ P,
+                                                        const double* __restrict__ recon,
+                                                        double* __restrict__ flux, double gamma, double inv_gm1) {
+  int b = blockIdx.x;
+#define MCFD_MERGED(SEGV)                                                                                         \
+  {                                                                                                               \
+    const int begin = g.seg_begin[SEGV], n = g.seg_begin[SEGV + 1] - begin;                                       \
+    const int nb = (n + (int)blockDim.x - 1) / (int)blockDim.x;                                                   \
+    if (b < nb) {                                                                                                 \
+      const int k = b * (int)blockDim.x + (int)threadIdx.x;                                                       \
+      if (k < n) flux_face<FLUX, SEGV, FIRST_ORDER, KERNEL_HLLC>(g, P, recon, flux, gamma, inv_gm1, begin + k, begin); \
+      return;                                                                                                     \
+    }                                                                                                             \
+    b -= nb;                                                                                                      \
+  }
+  MCFD_MERGED(SEG_FAR)
+  MCFD_MERGED(SEG_BCX)
+  MCFD_MERGED(SEG_VIN)
+  MCFD_MERGED(SEG_POUT)
+  MCFD_MERGED(SEG_WALL)
+  MCFD_MERGED(SEG_PERIODIC)
+  MCFD_MERGED(SEG_INTERIOR)
+#undef MCFD_MERGED
+}
+
 // --------------------------------------------------------------- time steps
 //
 // _stable_time_steps (solver.py:4132-4343), inviscid: per cell, the sum over
@@ -869,12 +905,11 @@ __global__ void k_time_step_finalize(DevStatus* st, double* dt_min, double time_
 
 // ------------------------------------------------------------------ launchers
 
-static inline int blocks_for(int n) { return (n + kBlock - 1) / kBlock; }
-
 
 cudaError_t launch_primitive(const DevGeom& g, const mcfd_config& cfg, const double* U, double* P,
                              cudaStream_t s) {
-  if (g.n_cells > 0) count_launch(), k_primitive<<<blocks_for(g.n_cells), kBlock, 0, s>>>(g.n_cells, U, P, cfg.gamma, g.status);
+  if (g.n_cells > 0)
+    count_launch(), k_primitive<<<seg_blocks(g.n_cells), seg_threads(g.n_cells), 0, s>>>(g.n_cells, U, P, cfg.gamma, g.status);
   return cudaGetLastError();
 }
 
@@ -892,6 +927,10 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
   }
   if constexpr (kFast || kMinRatio) {
     if (g.n_lim34 > 0 && g.tune_recon_split) {
+      // 64-thread blocks by default: RK3 step of the 1024^2 vortex 2,585 us
+      // against 2,591 / 2,617 with 128 / 256, of the 400^2 vortex 487 against
+      // 488 / 493; smaller meshes do not tell them apart
+      const int t = g.tune_recon_threads ? g.tune_recon_threads : 64;
       const int bs = (int)((4LL * g.n_lim34 + t - 1) / t);
       count_launch();
       switch (cfg.limiter) {
@@ -932,12 +971,31 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
   return cudaGetLastError();
 }
 
-// Boundary segments run on the side stream (when given) concurrently with
-// the interior faces; every face writes only its own flux row.
+// Meshes of more faces launch per segment, where each keeps its own register
+// count (the merged kernel's 76 to 84 against the interior's 64).  RK3 step
+// with one launch against one per segment: 2,970 faces (walls, far field) 130
+// / 161 us, 60,000 164 / 200, 240,000 452 / 495, 450,000 561 / 593; 625,000
+// faces of a periodic box 733 / 707.
+#ifndef MCFD_MERGED_FLUX_FACES
+#define MCFD_MERGED_FLUX_FACES 500000
+#endif
+constexpr int kMergedFluxFaces = MCFD_MERGED_FLUX_FACES;
+
+// Boundary segments of larger meshes run on the side stream (when given)
+// concurrently with the interior faces; every face writes only its own flux
+// row.
 template <int FLUX, bool FO, bool KH>
 static void flux_segments(const DevGeom& g, const double* P, const double* recon, double* flux,
                           double gamma, cudaStream_t s, const SideStream* side) {
   const double inv_gm1 = 1.0 / (gamma - 1.0);
+  if (g.n_flux > 0 && g.n_flux <= kMergedFluxFaces) {
+    const int t = seg_threads(g.n_flux);
+    int blocks = 0;
+    for (int k = 0; k < SEG_COUNT; ++k) blocks += (g.seg_begin[k + 1] - g.seg_begin[k] + t - 1) / t;
+    count_launch();
+    k_flux_merged<FLUX, FO, KH><<<blocks, t, 0, s>>>(g, P, recon, flux, gamma, inv_gm1);
+    return;
+  }
   const bool fork = side && side->stream && g.seg_begin[SEG_COUNT] > g.seg_begin[SEG_INTERIOR + 1];
   if (fork) {
     cudaEventRecord(side->fork, s);
@@ -997,7 +1055,7 @@ cudaError_t launch_gather(const DevGeom& g, const mcfd_config& cfg, const double
     else if (prog.t[1].kind == TERM_X_PLUS_DTR) shape = SHAPE_X_XDTR;
   }
   const bool extras = prog.visc_r || cfg.acceleration_x != 0.0 || cfg.acceleration_y != 0.0;
-  const int t = g.tune_gather_threads ? g.tune_gather_threads : kBlock;
+  const int t = g.tune_gather_threads ? g.tune_gather_threads : seg_threads(g.n_cells);
   const int b = (g.n_cells + t - 1) / t;
   const double ax = cfg.acceleration_x, ay = cfg.acceleration_y;
   count_launch();
@@ -1033,7 +1091,7 @@ cudaError_t launch_time_steps(const DevGeom& g, const mcfd_config& cfg, const do
                               double* dt_cells, double* dt_min, double time_limit,
                               cudaStream_t s) {
   if (g.n_cells > 0)
-    count_launch(), k_time_steps<<<blocks_for(g.n_cells), kBlock, 0, s>>>(g, P, cfg.gamma, cfg.cfl, dt_cells,
+    count_launch(), k_time_steps<<<seg_blocks(g.n_cells), seg_threads(g.n_cells), 0, s>>>(g, P, cfg.gamma, cfg.cfl, dt_cells,
                                                           dt_min != nullptr,
                                                           cfg.viscosity_model ? g.visc_diff : nullptr);
   if (dt_min) count_launch(), k_time_step_finalize<<<1, 1, 0, s>>>(g.status, dt_min, time_limit);
