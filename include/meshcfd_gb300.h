@@ -442,8 +442,10 @@ int mcfd_lusgs_apply(mcfd_geom* geom, const double* v, double* x, void* stream);
  * windows of up to 32 levels with a block barrier per level and a cluster
  * barrier per window (each block recomputes the rows of other bands its own
  * rows depend on inside the window; a plan that does not fit shared memory
- * takes engine 2).  0 restores the defaults (wide_level 16384, engine 9
- * where the device runs clusters of 16, else 7, else 2); 7, 8, 9 or 16
+ * takes engine 2).  0 restores the defaults: wide_level 16384 and, where no
+ * level is wider and the rows fit its plan, one pipeline of bands on a
+ * cluster of 16 or 8 blocks; otherwise engine 9 where the device runs
+ * clusters of 16, else 7, else 2; 7, 8, 9 or 16
  * returns MCFD_E_UNSUPPORTED where the device cannot run that cluster size.
  * Results do not depend on it.  No counterpart in the reference. */
 int mcfd_implicit_set_sweep(mcfd_geom* geom, int32_t wide_level, int32_t engine);

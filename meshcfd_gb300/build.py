@@ -35,6 +35,7 @@ UNITS = [
     ("mcfd_kernels_fma.cu", ["-fmad=true"]),
     ("mcfd_kernels_common.cu", ["-fmad=false"]),
     ("mcfd_implicit.cu", ["-fmad=false"]),
+    ("mcfd_pipeline.cu", ["-fmad=false"]),
     ("mcfd_jvp.cu", ["-fmad=false"]),
     ("mcfd_vjp.cu", ["-fmad=true"]),
     ("mcfd_parabolic.cu", ["-fmad=false"]),

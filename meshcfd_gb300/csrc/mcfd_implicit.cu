@@ -7,9 +7,8 @@
 //   the forward solve (D+L) y = v and backward solve (D+U) x = D y run over
 //   level sets of the natural-cell-order dependency graph, so the
 //   preconditioner is exactly the reference's (only independent rows run
-//   concurrently): runs of narrow levels in one block that barriers between
-//   levels and keeps the latest solutions in a shared-memory ring, wide
-//   levels one grid launch each;
+//   concurrently): runs of narrow levels on one thread-block cluster or in
+//   one block (mcfd_pipeline.cu by default), wide levels one grid launch each;
 // * the matrix-free operator v -> v - dt [R1(u + eps s v) - R1(u)] / (eps s)
 //   (_matrix_free_implicit_operator, solver.py:1532-1567);
 // * restarted GMRES(m) as the reference drives SciPy's gmres
@@ -1233,6 +1232,18 @@ cudaError_t implicit_set_wide_level(ImplicitState& st, int wide, int engine) {
   sweep_schedule(st.bwd, st.wide_level);
   free_windows(st.fwd.win);
   free_windows(st.bwd.win);
+  pipeline_free(st.fwd.pipe);
+  pipeline_free(st.bwd.pipe);
+  if (e == cudaSuccess && engine == 0 && st.pipeline_blocks > 0) {
+    e = pipeline_plan(st.fwd, st.bwd, st.n_cells, st.pipeline_blocks);
+    if (st.fwd.pipe.ok && st.bwd.pipe.ok) st.engine = kSweepPipeline;
+    if (e == cudaSuccess && st.engine == kSweepPipeline && st.prepared) {  // the new stage has no values yet
+      e = cudaDeviceSynchronize();  // the assembly may have run on any stream
+      if (e == cudaSuccess) e = pipeline_values(st.fwd, nullptr);
+      if (e == cudaSuccess) e = pipeline_values(st.bwd, nullptr);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+    }
+  }
   if (st.engine == kSweepWindow8 || st.engine == kSweepWindow16) {
     const int nc = st.engine == kSweepWindow16 ? 16 : 8;
     if (e == cudaSuccess) e = plan_windows(st.fwd, st.n_cells, nc);
@@ -1542,9 +1553,10 @@ cudaError_t implicit_build(ImplicitState& st, const ImplicitTopology& t) {
                                                  (int)kRingBytes);
   // Measured on the 512 x 256 bump (767 levels of at most 256 rows), one
   // LU-SGS application takes 3.20 ms in one block with per-row waits, 4.46 /
-  // 4.82 ms in a cluster of 8 / 16 sharing every solution, and 1.82 / 1.25 ms
-  // in the windowed band sweep on a cluster of 8 / 16, the default where the
-  // device runs it (set after the cluster checks below).
+  // 4.82 ms in a cluster of 8 / 16 sharing every solution, 1.82 / 1.25 ms in
+  // the windowed band sweep on a cluster of 8 / 16, and 0.74 ms in the
+  // pipelined band sweep, the default where the device runs it and it can be
+  // planned (after the cluster checks below).
   st.engine = kDefaultEngine;
   st.chunk_rows = kDefaultEngine == kSweepDataflowComponents ? 8 : kFlowChunk;
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_lusgs_dataflow<512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1604,6 +1616,7 @@ cudaError_t implicit_build(ImplicitState& st, const ImplicitTopology& t) {
   st.window8_ok = e == cudaSuccess && window_fits(k_lusgs_window<8>, 8);
   st.window16_ok = e == cudaSuccess && window_fits(k_lusgs_window<16>, 16);
   cudaGetLastError();
+  st.pipeline_blocks = e != cudaSuccess ? 0 : pipeline_available(16) ? 16 : pipeline_available(8) ? 8 : 0;
   st.default_engine = st.window16_ok ? kSweepWindow16 : (st.window8_ok ? kSweepWindow8 : kDefaultEngine);
   if (e == cudaSuccess) e = implicit_set_wide_level(st, 0, 0);
   if (e == cudaSuccess) {
@@ -1639,6 +1652,8 @@ void implicit_free(ImplicitState& st) {
   st.owned.clear();
   free_windows(st.fwd.win);
   free_windows(st.bwd.win);
+  pipeline_free(st.fwd.pipe);
+  pipeline_free(st.bwd.pipe);
   if (st.cycle_host) cudaFreeHost(st.cycle_host);
   st.cycle_host = nullptr;
 }
@@ -1664,6 +1679,8 @@ cudaError_t implicit_assemble(ImplicitState& st, const double* P, const double* 
     k_pack_rows<<<blocks_for(st.n_cells), kBlock, 0, s>>>(st.n_cells, pl->pos_cell, pl->ent_ptr, pl->ent_val,
                                                           st.rval, st.diag, st.dclamp, pl->pk_val, pl->pk_diag,
                                                           pl->pk_dc, pl->pk_row);
+    const cudaError_t e = pipeline_values(*pl, s);
+    if (e != cudaSuccess) return e;
   }
   return cudaGetLastError();
 }
@@ -1754,6 +1771,7 @@ static cudaError_t sweep(const SweepPlan& pl, const ImplicitState& st, const dou
 }
 
 cudaError_t lusgs_apply(ImplicitState& st, const double* v, double* x, cudaStream_t s) {
+  if (st.engine == kSweepPipeline) return pipeline_apply(st.fwd, st.bwd, v, x, st.status, s);
   cudaError_t e = sweep(st.fwd, st, v, st.tmp, 0, s);  // (D + L) y = v
   if (e == cudaSuccess) e = sweep(st.bwd, st, st.tmp, x, 1, s);  // (D + U) x = D y
   return e;

@@ -54,7 +54,8 @@ enum SweepEngine {
   kSweepWindow8 = 7,   // cluster of 8 blocks owning bands of cells, windows of levels (SweepWindows)
   kSweepCluster8 = 8,
   kSweepWindow16 = 9,  // the same with 16 blocks
-  kSweepCluster16 = 16
+  kSweepCluster16 = 16,
+  kSweepPipeline = 32  // cluster of blocks owning bands of cells, one pipeline (SweepPipeline); the default where planned
 };
 
 // The windowed band sweep of one plan for a cluster of nc blocks.  Block k
@@ -87,6 +88,18 @@ struct SweepWindows {
   std::vector<void*> owned;
 };
 
+// The pipelined band sweep of one plan (mcfd_pipeline.cu, planned by
+// mcfd_pipeline_plan.h): the staged rows in chunks of 64 by field, and per
+// band its first chunk, rows, externals and steps.
+struct SweepPipeline {
+  bool ok = false;  // planned for the current schedule
+  int nc = 0, groups = 0, n_padded = 0;
+  double* stage = nullptr;
+  int *chunk0 = nullptr, *rows = nullptr, *externals = nullptr, *step0 = nullptr, *steps = nullptr;
+  int *pos = nullptr, *cell = nullptr, *dest = nullptr;  // [n_padded], destinations [n_padded][4]
+  std::vector<void*> owned;
+};
+
 struct SweepPlan {
   int n_levels = 0;
   int* level_ptr = nullptr;  // [n_levels + 1] positions
@@ -110,6 +123,7 @@ struct SweepPlan {
   // host copies of the topology for planning the windowed sweep
   std::vector<int> host_pos_cell, host_ent_ptr, host_ent_pos;
   SweepWindows win;
+  SweepPipeline pipe;
   // chunks of at most 32 consecutive positions inside one level (start,
   // rows), for the dataflow sweep; chunk_ptr[l] = first chunk of level l
   int2* chunks = nullptr;
@@ -150,6 +164,7 @@ struct ImplicitState {
   int default_engine = kSweepDataflow;  // the fastest engine the device runs
   int chunk_rows = 32;  // rows per chunk of the per-row-wait sweeps
   bool cluster8_ok = false, cluster16_ok = false, window8_ok = false, window16_ok = false;
+  int pipeline_blocks = 0;  // cluster size of the pipelined sweep (0: the device runs none)
   DevStatus* status = nullptr;  // the geometry's status word (sweep time-outs)
   // values and vectors (device)
   double *coef = nullptr, *bterm = nullptr, *diag = nullptr, *dclamp = nullptr, *rval = nullptr;
@@ -188,6 +203,15 @@ enum GmresResult { GMRES_OK = 0, GMRES_NOT_CONVERGED = 1, GMRES_BREAKDOWN = 2, G
 using ResidualFn = std::function<cudaError_t(const double* U, double* R, cudaStream_t s)>;
 using MatvecFn = std::function<cudaError_t(const double* v, double* out, cudaStream_t s)>;
 
+// the pipelined band sweep: whether the device runs a cluster of nc such
+// blocks; planning (ok stays false where the schedule does not fit it); the
+// rows' values after an assembly; both sweeps of one application
+bool pipeline_available(int nc);
+void pipeline_free(SweepPipeline& p);
+cudaError_t pipeline_plan(SweepPlan& fwd, SweepPlan& bwd, int C, int nc);
+cudaError_t pipeline_values(SweepPlan& pl, cudaStream_t s);
+cudaError_t pipeline_apply(SweepPlan& fwd, SweepPlan& bwd, const double* v, double* x, DevStatus* status,
+                           cudaStream_t s);
 cudaError_t implicit_build(ImplicitState& st, const ImplicitTopology& t);
 void implicit_free(ImplicitState& st);
 cudaError_t implicit_assemble(ImplicitState& st, const double* P, const double* area, const double* dt,
