@@ -24,6 +24,7 @@
 
 #include "mcfd_device.cuh"
 #include "mcfd_implicit.h"
+#include "mcfd_reduce.cuh"
 #include "mcfd_window_plan.h"
 
 namespace cg = cooperative_groups;
@@ -825,12 +826,12 @@ __global__ void __launch_bounds__(kBlock) k_dot_partial(long long n, const doubl
   if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
 }
 
-__global__ void k_dot_final(int blocks, const double* __restrict__ partials, double* out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partials[b];
-    out[0] = s;
-  }
+// The block sums of a sum of squares in block order (ordered_sum_warp: the
+// sequential loop's bits; 32 us as one thread's loop, 8 us so).  Every
+// product these kernels reduce is a square, as the ordered sum needs.
+__global__ void __launch_bounds__(kBlock) k_dot_final(int blocks, const double* __restrict__ partials, double* out) {
+  __shared__ double sh[kRedBlocks];
+  ordered_sums_block(partials, blocks, 1, sh, out);
 }
 
 // Newton equation of the implicit step (solver.py:1415-1426):
@@ -946,11 +947,6 @@ __global__ void k_candidate(int C, const double* __restrict__ U, const double* _
   if (i < 4 * C) out[i] = U[i] + (damping * dx[i]) * s.v[i & 3];
 }
 
-__global__ void k_axpy(long long n, double a, const double* __restrict__ x, double* __restrict__ y) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n) y[i] = y[i] + a * x[i];
-}
-
 // r = b - x
 __global__ void k_sub(long long n, const double* __restrict__ b, const double* __restrict__ x,
                       double* __restrict__ r) {
@@ -962,10 +958,14 @@ __global__ void k_sub(long long n, const double* __restrict__ b, const double* _
 
 // eps = sqrt(machine eps) * max(1, |u/s|) / |v|  (solver.py:1546-1561);
 // |u/s| = sqrt of the prepared sum of squares
-__global__ void k_fd_eps(const double* __restrict__ v_sumsq, const double* __restrict__ state_sumsq,
-                         double* eps_out) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    const double dn = sqrt_rn(v_sumsq[0]);
+// and |v|^2 from the block sums (k_dot_final), stored as well
+__global__ void __launch_bounds__(kBlock) k_fd_eps(int blocks, const double* __restrict__ partials,
+                                                   double* __restrict__ v_sumsq,
+                                                   const double* __restrict__ state_sumsq, double* eps_out) {
+  __shared__ double sh[kRedBlocks];
+  ordered_sums_block(partials, blocks, 1, sh, v_sumsq);
+  if (threadIdx.x == 0) {
+    const double dn = sqrt_rn(v_sumsq[0]);  // this thread's own store
     const double state_norm = sqrt_rn(state_sumsq[0]);
     const double fd = 1.4901161193847656e-08;  // math.sqrt(np.finfo(float).eps)
     eps_out[0] = (dn == 0.0) ? 0.0 : div_rn(fd * (state_norm > 1.0 ? state_norm : 1.0), dn);
@@ -1142,49 +1142,83 @@ __global__ void k_givens(GmresCycle* cyc, const double* __restrict__ hcol, doubl
   if (use_handle) cudaGraphSetConditional(handle, done ? 0u : 1u);
 }
 
-// vcur = basis[col]
-__global__ void k_take_column(const double* __restrict__ basis, long long n, const GmresCycle* cyc,
-                              double* __restrict__ vcur) {
-  const double* v = basis + (size_t)cyc->col * n;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    vcur[i] = v[i];
-}
-
-// basis[last + 1] = w * inv_h1 (w unscaled at breakdown)
-__global__ void k_next_basis(double* __restrict__ basis, long long n, const GmresCycle* cyc,
-                             const double* __restrict__ w) {
+// basis[last + 1] = w * inv_h1 (w unscaled at breakdown), also into vcur,
+// the vector the next Arnoldi step multiplies, with the block sums of its
+// square that the finite-difference step needs (k_dot_partial's order: the
+// grid is its kRedBlocks x kBlock).  The first vector of a cycle: last = -1.
+__global__ void __launch_bounds__(kBlock) k_next_basis(double* __restrict__ basis, long long n, const GmresCycle* cyc,
+                                                       const double* __restrict__ w, double* __restrict__ vcur,
+                                                       double* __restrict__ partials) {
+  __shared__ double sh[kBlock];
   double* v = basis + (size_t)(cyc->last + 1) * n;
   const int scale = !cyc->breakdown;
   const double inv = cyc->inv_h1;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    v[i] = scale ? w[i] * inv : w[i];
+  double acc = 0.0;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double x = scale ? w[i] * inv : w[i];
+    v[i] = x;
+    vcur[i] = x;
+    acc += x * x;
+  }
+  sh[threadIdx.x] = acc;
+  __syncthreads();
+  for (int k = kBlock / 2; k > 0; k >>= 1) {
+    if (threadIdx.x < k) sh[threadIdx.x] += sh[threadIdx.x + k];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
 }
 
-// start of a restart cycle: S = (|z|, 0, ...), basis[0] = z / |z|, cycle
-// counters reset; |z|^2 given on the device
+// start of a restart cycle: S = (|z|, 0, ...), cycle counters reset, the
+// scale of the first basis vector 1 / |z|; |z|^2, |b|^2 and |M b|^2 given on
+// the device.  ptol = |M b| min(1, atol / |b|), atol = tol |b|
+// (iterative.py, gmres).
 __global__ void k_cycle_start(GmresCycle* cyc, double* __restrict__ givens, int m, const double* __restrict__ zsq,
-                              int restart, double ptol, double* __restrict__ inv_out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double z = sqrt(zsq[0]);
+                              const double* __restrict__ bsq, const double* __restrict__ mbsq, double tol,
+                              int restart) {
   double* S = givens + 2 * m;
-  for (int k = 0; k <= m; ++k) S[k] = 0.0;
+  for (int k = threadIdx.x; k <= m; k += blockDim.x) S[k] = 0.0;
+  __syncwarp();
+  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  const double z = sqrt(zsq[0]), bnrm2 = sqrt(bsq[0]);
+  const double ratio = tol * bnrm2 / bnrm2;
   S[0] = z;
-  inv_out[0] = 1.0 / z;
   cyc->col = 0;
   cyc->last = -1;
   cyc->restart = restart;
   cyc->inner = 0;
   cyc->breakdown = 0;
   cyc->done = 0;
-  cyc->ptol = ptol;
+  cyc->ptol = sqrt(mbsq[0]) * (ratio < 1.0 ? ratio : 1.0);
   cyc->presid = 0.0;
-  cyc->inv_h1 = 1.0;
+  cyc->inv_h1 = 1.0 / z;
 }
 
-// x = x * alpha[0]
-__global__ void k_scale_dev(long long n, const double* __restrict__ alpha, double* __restrict__ x) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n) x[i] = x[i] * alpha[0];
+// x = ((x + y0 v0) + y1 v1) + ... over up to kCombine basis vectors
+constexpr int kCombine = 32;
+struct CombineArgs {
+  const double* basis;
+  long long n;
+  double* x;
+  int count;
+  double y[kCombine];
+};
+__global__ void __launch_bounds__(kBlock) k_combine(CombineArgs a) {
+  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  double s = a.x[i];
+  const double* v = a.basis + i;
+  int k = 0;
+  for (; k + 4 <= a.count; k += 4) {
+    const double v0 = v[0], v1 = v[a.n], v2 = v[2 * a.n], v3 = v[3 * a.n];
+    s = s + a.y[k] * v0;
+    s = s + a.y[k + 1] * v1;
+    s = s + a.y[k + 2] * v2;
+    s = s + a.y[k + 3] * v3;
+    v += 4 * a.n;
+  }
+  for (; k < a.count; ++k, v += a.n) s = s + a.y[k] * v[0];
+  a.x[i] = s;
 }
 
 }  // namespace
@@ -1195,7 +1229,7 @@ cudaError_t implicit_dot(ImplicitState& st, long long n, const double* x, const 
                          cudaStream_t s) {
   count_launch(2);
   k_dot_partial<<<kRedBlocks, kBlock, 0, s>>>(n, x, y, st.partials);
-  k_dot_final<<<1, 32, 0, s>>>(kRedBlocks, st.partials, out);
+  k_dot_final<<<1, kBlock, 0, s>>>(kRedBlocks, st.partials, out);
   return cudaGetLastError();
 }
 
@@ -1795,9 +1829,13 @@ cudaError_t fd_operator(ImplicitState& st, const ResidualFn& residual1, const do
                         cudaStream_t s) {
   const int C = st.n_cells;
   const long long N = 4LL * C;
-  cudaError_t e = implicit_dot(st, N, v, v, st.scalars + 0, s);
+  cudaError_t e = cudaSuccess;
   count_launch(3);
-  k_fd_eps<<<1, 32, 0, s>>>(st.scalars + 0, st.scalars + 8, st.scalars + 1);
+  if (!st.vv_partials) {  // an Arnoldi step's vector comes with its block sums
+    count_launch();
+    k_dot_partial<<<kRedBlocks, kBlock, 0, s>>>(N, v, v, st.partials);
+  }
+  k_fd_eps<<<1, kBlock, 0, s>>>(kRedBlocks, st.partials, st.scalars + 0, st.scalars + 8, st.scalars + 1);
   k_fd_perturb<<<blocks_for(N), kBlock, 0, s>>>(C, st.state, v, st.scalars + 1, st.scale_dev, st.up);
   if (e == cudaSuccess) e = cudaGetLastError();
   if (e == cudaSuccess) e = residual1(st.up, st.rp, s);
@@ -1832,11 +1870,9 @@ static cudaError_t ensure_gmres_basis(ImplicitState& st, int m) {
 static cudaError_t arnoldi_step(ImplicitState& st, const MatvecFn& matvec, int m, cudaGraphConditionalHandle handle,
                                 int use_handle, cudaStream_t s) {
   const long long N = 4LL * st.n_cells;
-  const int grid = (int)std::min<long long>(blocks_for(N), 152LL * 8);
-  count_launch();
-  k_take_column<<<grid, kBlock, 0, s>>>(st.basis, N, st.cycle, st.vcur);
-  cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = matvec(st.vcur, st.av, s);
+  st.vv_partials = true;
+  cudaError_t e = matvec(st.vcur, st.av, s);
+  st.vv_partials = false;
   if (e == cudaSuccess) e = lusgs_apply(st, st.av, st.w, s);
   if (e == cudaSuccess) {
     MgsArgs a{st.basis, N, st.w, st.cycle, st.hcol, m, st.mgs_partials};
@@ -1855,7 +1891,7 @@ static cudaError_t arnoldi_step(ImplicitState& st, const MatvecFn& matvec, int m
   if (e == cudaSuccess) {
     count_launch(2);
     k_givens<<<1, 32, 0, s>>>(st.cycle, st.hcol, st.hess, st.givens, m, handle, use_handle);
-    k_next_basis<<<grid, kBlock, 0, s>>>(st.basis, N, st.cycle, st.w);
+    k_next_basis<<<kRedBlocks, kBlock, 0, s>>>(st.basis, N, st.cycle, st.w, st.vcur, st.partials);
     e = cudaGetLastError();
   }
   return e;
@@ -1922,7 +1958,6 @@ int gmres_solve(ImplicitState& st, const MatvecFn& matvec, int matvec_key, const
                 int max_iter, int m, int* iterations, cudaStream_t s) {
   const long long N = 4LL * st.n_cells;
   cudaError_t e = cudaSuccess;
-  auto grid = [&](long long n) { return blocks_for(n); };
   if (ensure_gmres_basis(st, m) != cudaSuccess) return GMRES_CUDA;
   const bool graph = matvec_key >= 0 && ensure_inner_graph(st, matvec, matvec_key * 4096 + m, m);
   double* w = st.w;
@@ -1930,41 +1965,31 @@ int gmres_solve(ImplicitState& st, const MatvecFn& matvec, int matvec_key, const
   cudaMemsetAsync(x, 0, N * sizeof(double), s);
   int used = 0;
   *iterations = 0;
-  bool x_nonzero = false;
   std::vector<double> H, S;
   GmresCycle& cyc = *st.cycle_host;
+  // Each pass of the loop is one SciPy gmres call with maxiter = 1
+  // (iterative.py, gmres).  |b| and |M b| are the same in every one; the
+  // first starts from r = b, so M r = M b; later ones from the residual the
+  // call before ended with, which is above atol.
+  e = implicit_dot(st, N, b, b, st.scalars + 2, s);
+  const double bnrm2 = std::sqrt(host_scalar(st.scalars + 2, s, &e));
+  if (e != cudaSuccess) return GMRES_CUDA;
+  if (bnrm2 == 0.0) {
+    cudaMemcpyAsync(x, b, N * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    return GMRES_OK;
+  }
+  const double atol = tol * bnrm2;
+  if (bnrm2 < atol) return GMRES_OK;  // the residual of x = 0 already passes
+  const double* r = b;
   while (used < max_iter) {
     const int restart = std::min(m, max_iter - used);
-    // ---- one SciPy gmres call with maxiter=1 (iterative.py, gmres)
-    e = implicit_dot(st, N, b, b, st.scalars + 2, s);
-    const double bnrm2 = std::sqrt(host_scalar(st.scalars + 2, s, &e));
-    if (e != cudaSuccess) return GMRES_CUDA;
-    if (bnrm2 == 0.0) {
-      cudaMemcpyAsync(x, b, N * sizeof(double), cudaMemcpyDeviceToDevice, s);
-      return GMRES_OK;
-    }
-    const double atol = tol * bnrm2;
-    if (lusgs_apply(st, b, w, s) != cudaSuccess) return GMRES_CUDA;
-    e = implicit_dot(st, N, w, w, st.scalars + 3, s);
-    const double mb = std::sqrt(host_scalar(st.scalars + 3, s, &e));
-    double ptol = mb * std::min(1.0, atol / bnrm2);
-    double* r = st.basis;
-    if (x_nonzero) {
-      if (matvec(x, av, s) != cudaSuccess) return GMRES_CUDA;
-      count_launch();
-      k_sub<<<grid(N), kBlock, 0, s>>>(N, b, av, r);
-    } else {
-      cudaMemcpyAsync(r, b, N * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    }
-    e = implicit_dot(st, N, r, r, st.scalars + 4, s);
-    if (std::sqrt(host_scalar(st.scalars + 4, s, &e)) < atol) return GMRES_OK;
-    // v0 = psolve(r) / |psolve(r)|, S = (|psolve(r)|, 0, ...)
+    // v0 = M r / |M r|, S = (|M r|, 0, ...)
     if (lusgs_apply(st, r, w, s) != cudaSuccess) return GMRES_CUDA;
-    cudaMemcpyAsync(st.basis, w, N * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    e = implicit_dot(st, N, st.basis, st.basis, st.scalars + 5, s);
+    e = implicit_dot(st, N, w, w, st.scalars + (r == b ? 3 : 5), s);
     count_launch(2);
-    k_cycle_start<<<1, 32, 0, s>>>(st.cycle, st.givens, m, st.scalars + 5, restart, ptol, st.scalars + 6);
-    k_scale_dev<<<grid(N), kBlock, 0, s>>>(N, st.scalars + 6, st.basis);
+    k_cycle_start<<<1, 32, 0, s>>>(st.cycle, st.givens, m, st.scalars + (r == b ? 3 : 5), st.scalars + 2,
+                                   st.scalars + 3, tol, restart);
+    k_next_basis<<<kRedBlocks, kBlock, 0, s>>>(st.basis, N, st.cycle, w, st.vcur, st.partials);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return GMRES_CUDA;
     // ---- the inner loop: graph replay, or one step at a time from the host
@@ -1987,8 +2012,9 @@ int gmres_solve(ImplicitState& st, const MatvecFn& matvec, int matvec_key, const
     // back substitution (upper triangular in h[k][k]) on the host
     H.resize((size_t)(col + 1) * (m + 1));
     S.resize(3 * (size_t)m + 2);
-    e = cudaMemcpy(H.data(), st.hess, H.size() * sizeof(double), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(S.data(), st.givens, S.size() * sizeof(double), cudaMemcpyDeviceToHost);
+    e = cudaMemcpyAsync(H.data(), st.hess, H.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(S.data(), st.givens, S.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return GMRES_CUDA;
     auto h = [&](int c, int k) { return H[(size_t)c * (m + 1) + k]; };
     std::vector<double> y(S.begin() + 2 * m, S.begin() + 2 * m + col + 1);
@@ -2001,21 +2027,24 @@ int gmres_solve(ImplicitState& st, const MatvecFn& matvec, int matvec_key, const
       }
     }
     if (y[0] != 0.0) y[0] /= h(0, 0);
-    for (int k = 0; k <= col; ++k) {
+    for (int k = 0; k <= col; k += kCombine) {
+      CombineArgs a{st.basis + (size_t)k * N, N, x, std::min(kCombine, col + 1 - k), {}};
+      for (int j = 0; j < a.count; ++j) a.y[j] = y[k + j];
       count_launch();
-      k_axpy<<<grid(N), kBlock, 0, s>>>(N, y[k], st.basis + (size_t)k * N, x);
+      k_combine<<<blocks_for(N), kBlock, 0, s>>>(a);
     }
-    x_nonzero = true;
+    // the residual, kept in the (spent) first basis vector for the next cycle
     if (matvec(x, av, s) != cudaSuccess) return GMRES_CUDA;
     count_launch();
-    k_sub<<<grid(N), kBlock, 0, s>>>(N, b, av, st.tmp);
-    e = implicit_dot(st, N, st.tmp, st.tmp, st.scalars + 7, s);
+    k_sub<<<blocks_for(N), kBlock, 0, s>>>(N, b, av, st.basis);
+    e = implicit_dot(st, N, st.basis, st.basis, st.scalars + 7, s);
     const double rnorm = std::sqrt(host_scalar(st.scalars + 7, s, &e));
     if (e != cudaSuccess) return GMRES_CUDA;
     used += inner;
     *iterations = used;
     if (rnorm <= atol) return GMRES_OK;
     if (inner == 0) break;
+    r = st.basis;
   }
   return GMRES_NOT_CONVERGED;
 }
@@ -2045,7 +2074,7 @@ cudaError_t implicit_scaled_sumsq(ImplicitState& st, const double* U, ScaleVec s
                                   cudaStream_t s) {
   count_launch(2);
   k_scaled_sumsq_partial<<<kRedBlocks, kBlock, 0, s>>>(4LL * st.n_cells, U, scale, st.partials);
-  k_dot_final<<<1, 32, 0, s>>>(kRedBlocks, st.partials, out);
+  k_dot_final<<<1, kBlock, 0, s>>>(kRedBlocks, st.partials, out);
   return cudaGetLastError();
 }
 

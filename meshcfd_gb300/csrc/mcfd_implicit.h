@@ -169,6 +169,7 @@ struct ImplicitState {
   // values and vectors (device)
   double *coef = nullptr, *bterm = nullptr, *diag = nullptr, *dclamp = nullptr, *rval = nullptr;
   double *tmp = nullptr, *state = nullptr, *rate = nullptr, *up = nullptr, *rp = nullptr;
+  bool vv_partials = false;  // partials hold the block sums of the next operand's square (an Arnoldi step)
   double *w = nullptr, *av = nullptr, *vcur = nullptr, *partials = nullptr, *scalars = nullptr;
   // prepared operator: scales, |state / scale|^2 and the time steps live on
   // the device, so a captured GMRES step reads the current values

@@ -63,6 +63,6 @@ extern "C" int mcfd_residual_sumsq_noalloc(const double* R, int64_t n_cells, dou
   mcfd::count_launch(2);
   mcfd::k_sumsq_partial<<<mcfd::kSumsqBlocks, mcfd::kSumsqThreads, 0, s>>>(static_cast<int>(n_cells), R, scratch);
   if (cudaPeekAtLastError() != cudaSuccess) return MCFD_E_CUDA;
-  mcfd::k_sumsq_final<<<1, 32, 0, s>>>(mcfd::kSumsqBlocks, scratch, sums);
+  mcfd::k_sumsq_final<<<1, mcfd::kSumsqThreads, 0, s>>>(mcfd::kSumsqBlocks, scratch, sums);
   return cudaPeekAtLastError() == cudaSuccess ? MCFD_OK : MCFD_E_CUDA;
 }

@@ -678,12 +678,12 @@ __global__ void k_sum_partial(int n, const double* __restrict__ x, double* __res
   if (threadIdx.x == 0) partials[blockIdx.x] = sh[0];
 }
 
+// One warp: 32 strided sums and a shuffle tree (a fixed order).
 __global__ void k_sum_final(int blocks, const double* __restrict__ partials, double* out) {
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int b = 0; b < blocks; ++b) s += partials[b];
-    out[0] = s;
-  }
+  double s = 0.0;
+  for (int b = threadIdx.x; b < blocks; b += 32) s += partials[b];
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+  if (threadIdx.x == 0) out[0] = s;
 }
 
 // The interior segment runs on s; the boundary segments (periodic, wall,
