@@ -121,6 +121,8 @@ struct DevGeom {
   const int* vd_other;        // other cell, or -1 on diffusive boundary faces
   const double* vd_len;
   const double* vd_dist;      // raw distance (the kernel takes max(d, 1e-14))
+  const double2* visc_entry;  // [n_gradient + n_diffusive] weighted offsets of the gradient and ghost entries (workspace)
+  const double* visc_normal;  // [C][4] xx, xy, yy, 1 / det or 0 (workspace)
   const double* visc_diff;    // [C] diffusion sum of the last viscous time step (workspace)
   // launch shapes chosen by mcfd_autotune (0: the defaults)
   int tune_recon_threads, tune_flux_threads, tune_flux_faces, tune_gather_threads;
@@ -245,6 +247,7 @@ struct ViscousWork {
   double* r = nullptr;      // [C][4]
   double* diff = nullptr;   // [C]
 };
+cudaError_t launch_viscous_plan(const DevGeom& g, double2* entry, double* normal, cudaStream_t s);
 cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, const double* P, const ViscousWork& w,
                                     cudaStream_t s);
 cudaError_t launch_viscous_diffusion(const DevGeom& g, const mcfd_config& cfg, const double* P,

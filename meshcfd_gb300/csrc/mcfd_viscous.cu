@@ -3,14 +3,16 @@
 // * k_visc_cells: T = p / (rho R), mu (constant or Sutherland,
 //   solver.py:2721-2737), conductivity mu gamma R / ((gamma - 1) Pr), and the
 //   time step's effective diffusivity (solver.py:4257-4260);
+// * k_visc_plan (once per geometry): the weights and normal matrices of the
+//   gradients, which depend on the mesh alone;
 // * k_visc_gradients (per cell): weighted least-squares gradients of
 //   (u, v, T) (_kernels.py:163-205) over the cell's gradient entries in the
 //   reference's order, then its ghost entries on diffusive boundary faces
 //   (_viscous_gradients, solver.py:3615-3714);
-// * k_visc_faces: the averaged face flux on interior and periodic faces
-//   (_viscous_flux, solver.py:3717-3747);
-// * k_visc_boundary (per diffusive boundary face): the reference's boundary
-//   corrections of the face gradient and values (solver.py:3939-4114);
+// * k_visc_fluxes: the averaged face flux on interior and periodic faces
+//   (_viscous_flux, solver.py:3717-3747), and per diffusive boundary face the
+//   reference's boundary corrections of the face gradient and values
+//   (solver.py:3939-4114);
 // * k_visc_gather (per cell): derivative = 0 - D @ flux (D the SciPy CSR
 //   divergence, ascending face order), then the periodic and boundary terms
 //   in the reference's np.add.at / loop order;
@@ -110,6 +112,39 @@ __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, 
   return true;
 }
 
+// The mesh-only part of the least-squares gradients, once per geometry: per
+// entry (gradient entries, then the diffusive faces' ghost entries) the
+// weighted offset w d, w = 1 / max(|d|^2, 1e-300), and per cell the normal
+// matrix, accumulated in the entries' order, with the reciprocal of its
+// determinant (0 where the reference leaves the gradient zero).
+__global__ void __launch_bounds__(kBlock) k_visc_plan(DevGeom g, double2* __restrict__ entry,
+                                                      double* __restrict__ normal) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= g.n_cells) return;
+  double xx = 0.0, xy = 0.0, yy = 0.0;
+  auto add = [&](double2 d) {
+    const double r2 = d.x * d.x + d.y * d.y;
+    const double w = div_rn(1.0, r2 > 1e-300 ? r2 : 1e-300);
+    const double wx = w * d.x, wy = w * d.y;
+    xx += wx * d.x;
+    xy += wx * d.y;
+    yy += wy * d.y;
+    return make_double2(wx, wy);
+  };
+  for (int e = g.grad_ptr[c], e1 = g.grad_ptr[c + 1]; e < e1; ++e) entry[e] = add(g.grad_d[e]);
+  for (int i = g.vb_ptr[c], i1 = g.vb_ptr[c + 1]; i < i1; ++i) {
+    const int j = g.vb_j[i];
+    entry[(size_t)g.n_gradient + j] = add(g.diff_ghost[j]);
+  }
+  const double det = xx * yy - xy * xy;
+  const double xxyy = xx * yy;
+  const double inv = det > 1e-14 * (xxyy > 1e-300 ? xxyy : 1e-300) ? div_rn(1.0, det) : 0.0;
+  st4(normal + 4 * (size_t)c, St4{xx, xy, yy, inv});
+}
+
+// Bound by FP64 issue and the gathers' latency; the normal matrix and the
+// weights (11 of an entry's 26 FP64 operations and its division) come from
+// the plan: 32 us per launch on 44,849 cells before, 27 us now (the boundary cells' exterior states are what is left).
 __global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const double* __restrict__ P, Visc vs,
                                                            const double* __restrict__ cell,
                                                            double* __restrict__ grad) {
@@ -118,26 +153,19 @@ __global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const doub
   const St4 p = ld4(P + 4 * (size_t)c);
   const St4 cc = ld4(cell + 4 * (size_t)c);
   const double cv[3] = {p.b, p.c, cc.a};
-  double xx = 0.0, xy = 0.0, yy = 0.0, bx[3] = {0.0, 0.0, 0.0}, by[3] = {0.0, 0.0, 0.0};
-  auto add = [&](double dx, double dy, const double diff[3]) {
-    const double r2 = dx * dx + dy * dy;
-    const double w = div_rn(1.0, r2 > 1e-300 ? r2 : 1e-300);
-    const double wx = w * dx, wy = w * dy;
-    xx += wx * dx;
-    xy += wx * dy;
-    yy += wy * dy;
+  double bx[3] = {0.0, 0.0, 0.0}, by[3] = {0.0, 0.0, 0.0};
+  auto add = [&](double2 w, const double diff[3]) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      bx[k] += wx * diff[k];
-      by[k] += wy * diff[k];
+      bx[k] += w.x * diff[k];
+      by[k] += w.y * diff[k];
     }
   };
   for (int e = g.grad_ptr[c], e1 = g.grad_ptr[c + 1]; e < e1; ++e) {
     const int nb = g.grad_nb[e];
     const St4 q = ld4(P + 4 * (size_t)nb);
     const double diff[3] = {q.b - cv[0], q.c - cv[1], cell[4 * (size_t)nb] - cv[2]};
-    const double2 d = g.grad_d[e];
-    add(d.x, d.y, diff);
+    add(g.visc_entry[e], diff);
   }
   int bits = 0;
   for (int i = g.vb_ptr[c], i1 = g.vb_ptr[c + 1]; i < i1; ++i) {
@@ -175,39 +203,37 @@ __global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const doub
       }
     }
     const double diff[3] = {ghost[0] - cv[0], ghost[1] - cv[1], ghost[2] - cv[2]};
-    const double2 go = g.diff_ghost[j];
-    add(go.x, go.y, diff);
+    add(g.visc_entry[(size_t)g.n_gradient + j], diff);
   }
   if (bits) flag(g.status, bits, c);
   double out[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const double det = xx * yy - xy * xy;
-  const double xxyy = xx * yy;
-  if (det > 1e-14 * (xxyy > 1e-300 ? xxyy : 1e-300)) {
-    const double inv = div_rn(1.0, det);
+  const St4 m = ld4(g.visc_normal + 4 * (size_t)c);
+  if (icmp::gt0(m.d)) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      out[2 * k] = (bx[k] * yy - by[k] * xy) * inv;
-      out[2 * k + 1] = (by[k] * xx - bx[k] * xy) * inv;
+      out[2 * k] = (bx[k] * m.c - by[k] * m.b) * m.d;
+      out[2 * k + 1] = (by[k] * m.a - bx[k] * m.b) * m.d;
     }
   }
-  double* dst = grad + 6 * (size_t)c;
+  double2* dst = reinterpret_cast<double2*>(grad + 6 * (size_t)c);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) dst[k] = out[k];
+  for (int k = 0; k < 3; ++k) dst[k] = make_double2(out[2 * k], out[2 * k + 1]);
 }
 
-__global__ void __launch_bounds__(kBlock) k_visc_faces(DevGeom g, const double* __restrict__ P,
-                                                       const double* __restrict__ cell,
-                                                       const double* __restrict__ grad, double* __restrict__ flux) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int n_faces = g.seg_begin[SEG_PERIODIC + 1];  // interior, then periodic pairs
-  if (i >= n_faces) return;
+__device__ __forceinline__ void visc_face(const DevGeom& g, const double* __restrict__ P,
+                                          const double* __restrict__ cell, const double* __restrict__ grad,
+                                          double* __restrict__ flux, int i) {
   const int o = g.ff_lcell[i], nb = g.ff_rcell[i];
   const double2 n = g.ff_normal[i];
-  const double* go = grad + 6 * (size_t)o;
-  const double* gn = grad + 6 * (size_t)nb;
+  const double2* go = reinterpret_cast<const double2*>(grad + 6 * (size_t)o);
+  const double2* gn = reinterpret_cast<const double2*>(grad + 6 * (size_t)nb);
   double fg[6];
 #pragma unroll
-  for (int k = 0; k < 6; ++k) fg[k] = 0.5 * (go[k] + gn[k]);
+  for (int k = 0; k < 3; ++k) {
+    const double2 a = go[k], b = gn[k];
+    fg[2 * k] = 0.5 * (a.x + b.x);
+    fg[2 * k + 1] = 0.5 * (a.y + b.y);
+  }
   const St4 po = ld4(P + 4 * (size_t)o), pn = ld4(P + 4 * (size_t)nb);
   const St4 co = ld4(cell + 4 * (size_t)o), cn = ld4(cell + 4 * (size_t)nb);
   double out[4];
@@ -216,12 +242,9 @@ __global__ void __launch_bounds__(kBlock) k_visc_faces(DevGeom g, const double* 
   st4(flux + 4 * (size_t)i, St4{out[0], out[1], out[2], out[3]});
 }
 
-__global__ void __launch_bounds__(kBlock) k_visc_boundary(DevGeom g, const double* __restrict__ P, Visc vs,
-                                                          const double* __restrict__ cell,
-                                                          const double* __restrict__ grad,
-                                                          double* __restrict__ bflux) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= g.n_diffusive) return;
+__device__ __forceinline__ void visc_boundary(const DevGeom& g, const double* __restrict__ P, const Visc& vs,
+                                              const double* __restrict__ cell, const double* __restrict__ grad,
+                                              double* __restrict__ bflux, int j) {
   const int o = g.diff_owner[j];
   const double2 nn = g.diff_normal[j];
   const double nx = nn.x, ny = nn.y;
@@ -328,6 +351,23 @@ __global__ void __launch_bounds__(kBlock) k_visc_boundary(DevGeom g, const doubl
   st4(bflux + 4 * (size_t)j, St4{out[0], out[1], out[2], out[3]});
 }
 
+// The face fluxes: the diffusive boundary faces' blocks first (their chain of
+// divisions and Sutherland's power is the longest), then interior and
+// periodic faces.
+__global__ void __launch_bounds__(kBlock) k_visc_fluxes(DevGeom g, const double* __restrict__ P, Visc vs,
+                                                        const double* __restrict__ cell,
+                                                        const double* __restrict__ grad, double* __restrict__ flux,
+                                                        double* __restrict__ bflux, int boundary_blocks) {
+  const int b = (int)blockIdx.x;
+  if (b < boundary_blocks) {
+    const int j = b * blockDim.x + threadIdx.x;
+    if (j < g.n_diffusive) visc_boundary(g, P, vs, cell, grad, bflux, j);
+  } else {
+    const int i = (b - boundary_blocks) * blockDim.x + threadIdx.x;
+    if (i < g.seg_begin[SEG_PERIODIC + 1]) visc_face(g, P, cell, grad, flux, i);
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) k_visc_gather(DevGeom g, const double* __restrict__ flux,
                                                         const double* __restrict__ bflux, double* __restrict__ r) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,13 +441,19 @@ cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, co
                                     cudaStream_t s) {
   const Visc vs = visc_of(cfg);
   const int C = g.n_cells, nf = g.seg_begin[SEG_PERIODIC + 1];
-  count_launch(4 + (g.n_diffusive > 0));
-  k_visc_cells<<<blocks_for(C), kBlock, 0, s>>>(g, P, vs, w.cell);
-  k_visc_gradients<<<blocks_for(C), kBlock, 0, s>>>(g, P, vs, w.cell, w.grad);
-  if (nf > 0) k_visc_faces<<<blocks_for(nf), kBlock, 0, s>>>(g, P, w.cell, w.grad, w.flux);
-  if (g.n_diffusive > 0)
-    k_visc_boundary<<<blocks_for(g.n_diffusive), kBlock, 0, s>>>(g, P, vs, w.cell, w.grad, w.bflux);
-  k_visc_gather<<<blocks_for(C), kBlock, 0, s>>>(g, w.flux, w.bflux, w.r);
+  const int t = seg_threads(C) < kBlock ? seg_threads(C) : kBlock, tf = seg_threads(nf) < kBlock ? seg_threads(nf) : kBlock;
+  const int bb = (g.n_diffusive + tf - 1) / tf, fb = (nf + tf - 1) / tf;
+  count_launch(4);
+  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell);
+  k_visc_gradients<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, w.grad);
+  if (bb + fb > 0) k_visc_fluxes<<<bb + fb, tf, 0, s>>>(g, P, vs, w.cell, w.grad, w.flux, w.bflux, bb);
+  k_visc_gather<<<(C + t - 1) / t, t, 0, s>>>(g, w.flux, w.bflux, w.r);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_viscous_plan(const DevGeom& g, double2* entry, double* normal, cudaStream_t s) {
+  count_launch();
+  k_visc_plan<<<blocks_for(g.n_cells), kBlock, 0, s>>>(g, entry, normal);
   return cudaGetLastError();
 }
 
@@ -415,9 +461,10 @@ cudaError_t launch_viscous_diffusion(const DevGeom& g, const mcfd_config& cfg, c
                                      const ViscousWork& w, cudaStream_t s) {
   const Visc vs = visc_of(cfg);
   const int C = g.n_cells;
+  const int t = seg_threads(C) < kBlock ? seg_threads(C) : kBlock;
   count_launch(2);
-  k_visc_cells<<<blocks_for(C), kBlock, 0, s>>>(g, P, vs, w.cell);
-  k_visc_diffusion<<<blocks_for(C), kBlock, 0, s>>>(g, w.cell, w.diff);
+  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell);
+  k_visc_diffusion<<<(C + t - 1) / t, t, 0, s>>>(g, w.cell, w.diff);
   return cudaGetLastError();
 }
 
