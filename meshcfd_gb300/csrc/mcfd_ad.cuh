@@ -58,7 +58,7 @@ __device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, const Dual<N>& b)
   Dual<N> r;
   r.v = a.v * b.v;
 #pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = ia::fma_rn(a.d[k], b.v, a.v * b.d[k]);
   return r;
 }
 template <int N>
@@ -67,7 +67,33 @@ __device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, const Dual<N>& b)
   const double ib = div_rn(1.0, b.v);
   r.v = a.v * ib;
 #pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = (a.d[k] - r.v * b.d[k]) * ib;
+  for (int k = 0; k < N; ++k) r.d[k] = ia::fma_rn(-r.v, b.d[k], a.d[k]) * ib;
+  return r;
+}
+// A constant operand has no tangent.  As a Dual it would have zero ones, and
+// the compiler may not drop the products and sums with them (x 0 is not 0
+// for every x): two of the three FP64 operations per tangent of a product
+// with a face normal or a gas constant, half of the Roe flux's.
+template <int N>
+__device__ __forceinline__ Dual<N> operator*(const Dual<N>& a, double b) {
+  Dual<N> r;
+  r.v = a.v * b;
+#pragma unroll
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b;
+  return r;
+}
+template <int N>
+__device__ __forceinline__ Dual<N> operator*(double a, const Dual<N>& b) {
+  return b * a;
+}
+template <int N>
+__device__ __forceinline__ Dual<N> operator/(const Dual<N>& a, double b) {
+  return a * div_rn(1.0, b);
+}
+template <int N>
+__device__ __forceinline__ Dual<N> operator-(const Dual<N>& a, double b) {
+  Dual<N> r = a;
+  r.v = a.v - b;
   return r;
 }
 template <int N>
@@ -119,28 +145,28 @@ __device__ __forceinline__ S4<T> prim(const S4<T>& U, double gamma) {
   T rho = U.a;
   T ux = U.b / rho;
   T uy = U.c / rho;
-  T p = T(gamma - 1.0) * (U.d - T(0.5) * (U.b * U.b + U.c * U.c) / rho);
+  T p = (gamma - 1.0) * (U.d - 0.5 * (U.b * U.b + U.c * U.c) / rho);
   return S4<T>{rho, ux, uy, p};
 }
 
 // euler.physical_flux
 template <typename T>
 __device__ __forceinline__ void physical(const S4<T>& q, double nx, double ny, double gamma, T F[4], T U[4]) {
-  T energy = q.d / T(gamma - 1.0) + T(0.5) * q.a * (q.b * q.b + q.c * q.c);
-  T un = q.b * T(nx) + q.c * T(ny);
+  T energy = q.d / (gamma - 1.0) + 0.5 * q.a * (q.b * q.b + q.c * q.c);
+  T un = q.b * nx + q.c * ny;
   U[0] = q.a;
   U[1] = q.a * q.b;
   U[2] = q.a * q.c;
   U[3] = energy;
   F[0] = q.a * un;
-  F[1] = U[1] * un + q.d * T(nx);
-  F[2] = U[2] * un + q.d * T(ny);
+  F[1] = U[1] * un + q.d * nx;
+  F[2] = U[2] * un + q.d * ny;
   F[3] = (energy + q.d) * un;
 }
 
 template <typename T>
 __device__ __forceinline__ T sound(const S4<T>& q, double gamma) {
-  return sqrt(T(gamma) * q.d / q.a);
+  return sqrt(gamma * q.d / q.a);
 }
 
 template <typename T>
@@ -149,11 +175,11 @@ __device__ __forceinline__ void rusanov(const S4<T>& L, const S4<T>& R, double n
   T FL[4], UL[4], FR[4], UR[4];
   physical(L, nx, ny, gamma, FL, UL);
   physical(R, nx, ny, gamma, FR, UR);
-  T sl = fabs(L.b * T(nx) + L.c * T(ny)) + sound(L, gamma);
-  T sr = fabs(R.b * T(nx) + R.c * T(ny)) + sound(R, gamma);
+  T sl = fabs(L.b * nx + L.c * ny) + sound(L, gamma);
+  T sr = fabs(R.b * nx + R.c * ny) + sound(R, gamma);
   T s = val(sl) >= val(sr) ? sl : sr;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) out[k] = T(0.5) * ((FL[k] + FR[k]) - s * (UR[k] - UL[k]));
+  for (int k = 0; k < 4; ++k) out[k] = 0.5 * ((FL[k] + FR[k]) - s * (UR[k] - UL[k]));
 }
 
 template <typename T, bool KERNEL_BRANCHES>
@@ -161,7 +187,7 @@ __device__ __forceinline__ void hllc(const S4<T>& L, const S4<T>& R, double nx, 
   T FL[4], UL[4], FR[4], UR[4];
   physical(L, nx, ny, gamma, FL, UL);
   physical(R, nx, ny, gamma, FR, UR);
-  T unl = L.b * T(nx) + L.c * T(ny), unr = R.b * T(nx) + R.c * T(ny);
+  T unl = L.b * nx + L.c * ny, unr = R.b * nx + R.c * ny;
   T cl = sound(L, gamma), cr = sound(R, gamma);
   T wl = tmin(unl - cl, unr - cr);
   T wr = tmax(unl + cl, unr + cr);
@@ -191,8 +217,8 @@ __device__ __forceinline__ void hllc(const S4<T>& L, const S4<T>& R, double nx, 
   T un = left ? unl : unr;
   T wave = left ? wl : wr;
   T factor = q.a * (wave - un) / (wave - contact);
-  T sux = q.b + (contact - un) * T(nx);
-  T suy = q.c + (contact - un) * T(ny);
+  T sux = q.b + (contact - un) * nx;
+  T suy = q.c + (contact - un) * ny;
   T se = factor * (U[3] / q.a + (contact - un) * (contact + q.d / (q.a * (wave - un))));
   T star[4] = {factor, factor * sux, factor * suy, se};
 #pragma unroll
@@ -208,55 +234,55 @@ __device__ __forceinline__ void roe(const S4<T>& L, const S4<T>& R, double nx, d
   T den = rl + rr;
   T vx = (rl * L.b + rr * R.b) / den;
   T vy = (rl * L.c + rr * R.c) / den;
-  T H = (rl * (L.d / L.a + T(0.5) * (L.b * L.b + L.c * L.c)) + rr * (R.d / R.a + T(0.5) * (R.b * R.b + R.c * R.c))) / den;
-  T un = vx * T(nx) + vy * T(ny);
-  T ut = vx * T(-ny) + vy * T(nx);
-  T c2 = T(gamma - 1.0) * (H - T(0.5) * (vx * vx + vy * vy));
+  T H = (rl * (L.d / L.a + 0.5 * (L.b * L.b + L.c * L.c)) + rr * (R.d / R.a + 0.5 * (R.b * R.b + R.c * R.c))) / den;
+  T un = vx * nx + vy * ny;
+  T ut = vx * (-ny) + vy * nx;
+  T c2 = (gamma - 1.0) * (H - 0.5 * (vx * vx + vy * vy));
   T c = sqrt(c2);
   T ravg = rl * rr;
-  T unl = L.b * T(nx) + L.c * T(ny), unr = R.b * T(nx) + R.c * T(ny);
-  T utl = L.b * T(-ny) + L.c * T(nx), utr = R.b * T(-ny) + R.c * T(nx);
+  T unl = L.b * nx + L.c * ny, unr = R.b * nx + R.c * ny;
+  T utl = L.b * (-ny) + L.c * nx, utr = R.b * (-ny) + R.c * nx;
   T dr = R.a - L.a, dun = unr - unl, dut = utr - utl, dp = R.d - L.d;
-  T am = (dp - ravg * c * dun) / (T(2.0) * c2);
-  T ap = (dp + ravg * c * dun) / (T(2.0) * c2);
+  T am = (dp - ravg * c * dun) / (2.0 * c2);
+  T ap = (dp + ravg * c * dun) / (2.0 * c2);
   T ac = dr - dp / c2;
   T as = ravg * dut;
   T lam[4] = {un - c, un, un, un + c};
-  T fix = T(0.1) * c;
+  T fix = 0.1 * c;
   T strength[4] = {am, ac, as, ap};
   T w[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     T a = fabs(lam[j]);
-    if (val(a) < val(fix)) a = T(0.5) * (a * a / fix + fix);
+    if (val(a) < val(fix)) a = 0.5 * (a * a / fix + fix);
     w[j] = a * strength[j];
   }
   T d0 = w[0] + w[1] + w[3];
   T d1 = (un - c) * w[0] + un * w[1] + (un + c) * w[3];
   T d2 = ut * (w[0] + w[1] + w[3]) + w[2];
-  T d3 = (H - un * c) * w[0] + T(0.5) * (un * un + ut * ut) * w[1] + ut * w[2] + (H + un * c) * w[3];
-  T diss[4] = {d0, d1 * T(nx) - d2 * T(ny), d1 * T(ny) + d2 * T(nx), d3};
+  T d3 = (H - un * c) * w[0] + 0.5 * (un * un + ut * ut) * w[1] + ut * w[2] + (H + un * c) * w[3];
+  T diss[4] = {d0, d1 * nx - d2 * ny, d1 * ny + d2 * nx, d3};
 #pragma unroll
-  for (int k = 0; k < 4; ++k) out[k] = T(0.5) * ((FL[k] + FR[k]) - diss[k]);
+  for (int k = 0; k < 4; ++k) out[k] = 0.5 * ((FL[k] + FR[k]) - diss[k]);
 }
 
 template <typename T>
 __device__ __forceinline__ S4<T> far_field(const S4<T>& in, const S4<T>& far, double nx, double ny, double gamma) {
-  T ui = in.b * T(nx) + in.c * T(ny);
-  T uf = far.b * T(nx) + far.c * T(ny);
+  T ui = in.b * nx + in.c * ny;
+  T uf = far.b * nx + far.c * ny;
   T ci = sound(in, gamma), cf = sound(far, gamma);
   if (val(ui) <= -val(ci)) return far;
   if (val(ui) >= val(ci)) return in;
-  T out_inv = ui + T(2.0) * ci / T(gamma - 1.0);
-  T in_inv = uf - T(2.0) * cf / T(gamma - 1.0);
-  T vb = T(0.5) * (out_inv + in_inv);
-  T cb = T(0.25 * (gamma - 1.0)) * (out_inv - in_inv);
+  T out_inv = ui + 2.0 * ci / (gamma - 1.0);
+  T in_inv = uf - 2.0 * cf / (gamma - 1.0);
+  T vb = 0.5 * (out_inv + in_inv);
+  T cb = (0.25 * (gamma - 1.0)) * (out_inv - in_inv);
   const S4<T>& src = val(vb) < 0.0 ? far : in;
   T entropy = src.d / pow(src.a, gamma);
-  T rho = pow(cb * cb / (T(gamma) * entropy), 1.0 / (gamma - 1.0));
+  T rho = pow(cb * cb / (gamma * entropy), 1.0 / (gamma - 1.0));
   T p = entropy * pow(rho, gamma);
-  T vt = src.b * T(-ny) + src.c * T(nx);
-  return S4<T>{rho, vb * T(nx) + vt * T(-ny), vb * T(ny) + vt * T(nx), p};
+  T vt = src.b * (-ny) + src.c * nx;
+  return S4<T>{rho, vb * nx + vt * (-ny), vb * ny + vt * nx, p};
 }
 
 template <typename T>

@@ -212,6 +212,16 @@ inline int seg_threads(int n) {
   return n < 152 * 128 * 16 ? 128 : 256;
 }
 inline int seg_blocks(int n) { return (n + seg_threads(n) - 1) / seg_threads(n); }
+// Faces up to which one launch covers every face segment (k_flux_merged).
+// Meshes of more faces launch per segment, where each keeps its own register
+// count (the merged kernel's 76 to 84 against the interior's 64).  RK3 step
+// with one launch against one per segment: 2,970 faces (walls, far field) 130
+// / 161 us, 60,000 164 / 200, 240,000 452 / 495, 450,000 561 / 593; 625,000
+// faces of a periodic box 733 / 707.
+#ifndef MCFD_MERGED_FLUX_FACES
+#define MCFD_MERGED_FLUX_FACES 500000
+#endif
+constexpr int kMergedFluxFaces = MCFD_MERGED_FLUX_FACES;
 // flux launch shape with the autotuned threads / faces per thread, if any
 inline int flux_threads(const DevGeom& g, int n) {
   return g.tune_flux_threads && n >= 152 * g.tune_flux_threads ? g.tune_flux_threads : seg_threads(n);

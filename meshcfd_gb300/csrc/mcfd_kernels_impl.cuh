@@ -971,16 +971,6 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
   return cudaGetLastError();
 }
 
-// Meshes of more faces launch per segment, where each keeps its own register
-// count (the merged kernel's 76 to 84 against the interior's 64).  RK3 step
-// with one launch against one per segment: 2,970 faces (walls, far field) 130
-// / 161 us, 60,000 164 / 200, 240,000 452 / 495, 450,000 561 / 593; 625,000
-// faces of a periodic box 733 / 707.
-#ifndef MCFD_MERGED_FLUX_FACES
-#define MCFD_MERGED_FLUX_FACES 500000
-#endif
-constexpr int kMergedFluxFaces = MCFD_MERGED_FLUX_FACES;
-
 // Boundary segments of larger meshes run on the side stream (when given)
 // concurrently with the interior faces; every face writes only its own flux
 // row.
