@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(kBlock) k_vjp_face(DevGeom g, const double* __
     R = S{seed<8>(qR.a, 4), seed<8>(qR.b, 5), seed<8>(qR.c, 6), seed<8>(qR.d, 7)};
   } else if (SEG == SEG_WALL) {
     const double2 wv = g.ff_wall_velocity[f - begin];
-    D8 un = (L.b - D8(wv.x)) * D8(n.x) + (L.c - D8(wv.y)) * D8(n.y);
-    R = S{L.a, L.b - D8(2.0) * un * D8(n.x), L.c - D8(2.0) * un * D8(n.y), L.d};
+    D8 un = (L.b - wv.x) * n.x + (L.c - wv.y) * n.y;
+    R = S{L.a, L.b - 2.0 * un * n.x, L.c - 2.0 * un * n.y, L.d};
   } else if (SEG == SEG_VIN) {
     const St4 x = ld4(g.ff_vin_state + 4 * (size_t)(f - begin));
     R = S{D8(x.a), D8(x.b), D8(x.c), D8(x.d)};
@@ -330,26 +330,37 @@ __global__ void __launch_bounds__(kBlock) k_vjp_face(DevGeom g, const double* __
   if (SEG == SEG_FAR && far_bar) st4(far_bar + 4 * (size_t)(f - begin), St4{bar[4], bar[5], bar[6], bar[7]});
 }
 
+// Limiter function of a cell's smallest ratio r >= 0 and its slope there
+// (both 1 and 0 where it is capped): every limiter is nondecreasing in r up to
+// its cap.
 template <int LIMITER>
-__device__ __forceinline__ double limiter_slope(double r) {
-  if (LIMITER <= 1) return icmp::lt(r, 1.0) ? 1.0 : 0.0;
+__device__ __forceinline__ double limiter_value(double r, double* slope) {
+  *slope = 0.0;
+  if (LIMITER <= 1) {
+    if (!icmp::lt_pos(r, 1.0)) return 1.0;
+    *slope = 1.0;
+    return r;
+  }
   if (LIMITER == 2) {
     if (!icmp::gt0(r)) return 0.0;
-    return icmp::lt(r, 1.0) ? div_rn(2.0, (1.0 + r) * (1.0 + r)) : 0.0;  // 2r / (1 + r) < 1 iff r < 1
+    if (!icmp::lt_pos(r, 1.0)) return 1.0;  // 2r / (1 + r) < 1 iff r < 1
+    const double i = div_rn(1.0, 1.0 + r);
+    *slope = 2.0 * i * i;
+    return 2.0 * r * i;
   }
   const double eps = 1e-12;
   const double N = r * r + 2.0 * r + eps, D = r * r + r + 2.0 + eps;
-  if (N > D) return 0.0;  // capped at 1
+  if (!icmp::lt_pos(N, D)) return 1.0;
   const double inv_D = div_rn(1.0, D);
-  return ((2.0 * r + 2.0) * D - N * (2.0 * r + 1.0)) * (inv_D * inv_D);
+  *slope = ((2.0 * r + 2.0) * D - N * (2.0 * r + 1.0)) * (inv_D * inv_D);
+  return N * inv_D;
 }
 
-// The cell reverse of one variable (the cell kernel's loop body): the
-// variable's gradient and extremes, limiter minimum and its first entry,
-// then the reverse of the face states, of the limiter and of the gradient.
-// One variable's state is live at a time (96 registers instead of 128 with
-// spills for all four at once), and its increments are kept for the reverse
-// instead of being recomputed.  NS > 0 compiles the cell for exactly NS
+// The cell reverse of one variable: the variable's gradient and extremes,
+// limiter minimum and its first entry, then the reverse of the face states, of
+// the limiter and of the gradient.  One thread takes one variable of a cell
+// (k_vjp_cell); its increments and slot adjoints are kept for the reverse
+// instead of being recomputed and read again.  NS > 0 compiles the cell for exactly NS
 // limiter entries (the cell order makes the count warp-uniform, so a warp of
 // triangles issues no FP64 work for a fourth entry); NS = 0 handles any
 // count, keeping the first four increments.
@@ -457,14 +468,15 @@ __device__ __forceinline__ void vjp_cell_variable(const DevGeom& g, const double
     if (icmp::lt(q, lo)) { lo = q; lo_e = e; }
     if (icmp::lt(hi, q)) { hi = q; hi_e = e; }
   }
-  // phi = min over entries of f(max(r, 0)) and its first entry, from the
-  // three candidates (largest positive increment, most negative, first
-  // entry in the tolerance band)
+  // phi = min over entries of f(max(r, 0)), the limiter at the smallest ratio:
+  // that of the largest positive increment, of the most negative one, or 1 in
+  // the tolerance band (correctly rounded division is monotone); equal ratios
+  // go to the first entry
   const double tol = limiter_tolerance(pv);
   double pmax = 0.0, nmin = 0.0;
   int ps = -1, ns = -1, fs = -1;
   constexpr int kCache = NS > 0 ? NS : 4;
-  double incs[kCache];
+  double incs[kCache], qbs[kCache];
   auto classify = [&](int s, double inc) {
     if (icmp::gt_pos(inc, tol)) {
       if (ps < 0 || icmp::lt(pmax, inc)) { pmax = inc; ps = s; }
@@ -479,6 +491,8 @@ __device__ __forceinline__ void vjp_cell_variable(const DevGeom& g, const double
     incs[k] = 0.0;
     if (NS > 0 || s0 + k < s1) {
       const double2 dd = g.lim_d[s0 + k];
+      qbs[k] = slot_bar[4 * (size_t)g.lim_slot[s0 + k] + v];
+      pb += qbs[k];
       incs[k] = mul_rn(gx, dd.x) + gy * dd.y;
       classify(s0 + k, incs[k]);
     }
@@ -486,28 +500,28 @@ __device__ __forceinline__ void vjp_cell_variable(const DevGeom& g, const double
   if (NS == 0) {
     for (int s = s0 + kCache; s < s1; ++s) {
       const double2 dd = g.lim_d[s];
+      pb += slot_bar[4 * (size_t)g.lim_slot[s] + v];
       classify(s, mul_rn(gx, dd.x) + gy * dd.y);
     }
   }
-  double phi = 1.0;
-  int arg = -1;
+  double r = 1.0, arg_inc = 1.0;
+  int arg = fs;
   {
-    const int cand[3] = {ps, ns, fs};
-    const double cinc[3] = {pmax, nmin, 0.0};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      if (cand[k] < 0) continue;
-      const double f = limiter_face_factor<LIMITER>(pv, cinc[k], lo, hi, tol);
-      if (icmp::lt_nonneg(f, phi) || (icmp::key(f) == icmp::key(phi) && arg >= 0 && cand[k] < arg)) {
-        phi = f;
-        arg = cand[k];
-      }
+    const double rp = div_rn(hi - pv, ps >= 0 ? pmax : 1.0), rn = div_rn(lo - pv, ns >= 0 ? nmin : -1.0);
+    if (ps >= 0) {
+      const double x = icmp::ge0(rp) ? rp : 0.0;
+      if (arg < 0 || icmp::lt_nonneg(x, r) || (icmp::key(x) == icmp::key(r) && ps < arg)) r = x, arg = ps, arg_inc = pmax;
+    }
+    if (ns >= 0) {
+      const double x = icmp::ge0(rn) ? rn : 0.0;
+      if (arg < 0 || icmp::lt_nonneg(x, r) || (icmp::key(x) == icmp::key(r) && ns < arg)) r = x, arg = ns, arg_inc = nmin;
     }
   }
+  double slope = 0.0;
+  const double phi = arg >= 0 ? limiter_value<LIMITER>(r, &slope) : 1.0;
   // reverse of Q_s = P + phi (G . r_s)
   double phib = 0.0, gxb = 0.0, gyb = 0.0;
-  auto face_reverse = [&](int s, double inc, const double2& dd) {
-    const double qb = slot_bar[4 * (size_t)g.lim_slot[s] + v];
+  auto face_reverse = [&](double qb, double inc, const double2& dd) {
     phib += qb * inc;
     const double qphi = mul_rn(qb, phi);
     gxb += qphi * dd.x;
@@ -515,41 +529,26 @@ __device__ __forceinline__ void vjp_cell_variable(const DevGeom& g, const double
   };
 #pragma unroll
   for (int k = 0; k < kCache; ++k)
-    if (NS > 0 || s0 + k < s1) face_reverse(s0 + k, incs[k], g.lim_d[s0 + k]);
+    if (NS > 0 || s0 + k < s1) face_reverse(qbs[k], incs[k], g.lim_d[s0 + k]);
   if (NS == 0) {
     for (int s = s0 + kCache; s < s1; ++s) {
       const double2 dd = g.lim_d[s];
-      face_reverse(s, mul_rn(gx, dd.x) + gy * dd.y, dd);
+      face_reverse(slot_bar[4 * (size_t)g.lim_slot[s] + v], mul_rn(gx, dd.x) + gy * dd.y, dd);
     }
   }
   // reverse of the limiter through its minimising entry
   double extb = 0.0;
   int ext_e = -1;
-  if (arg >= 0) {
+  if (arg >= 0 && arg != fs && icmp::gt0(r) && icmp::gt0(slope)) {
     const double2 dd = g.lim_d[arg];
-    const int k = arg - s0;
-    double inc = incs[0];
-#pragma unroll
-    for (int m = 1; m < kCache; ++m)
-      if (k == m) inc = incs[m];
-    if (NS == 0 && k >= kCache) inc = mul_rn(gx, dd.x) + gy * dd.y;
-    const bool pos = icmp::gt_pos(inc, tol), neg = icmp::neg_gt_pos(inc, tol);
-    if (pos || neg) {
-      const double num = pos ? hi - pv : lo - pv;
-      const double inv_inc = div_rn(1.0, inc);
-      const double r = num * inv_inc;
-      if (icmp::gt0(r)) {
-        const double rb = limiter_slope<LIMITER>(r) * phib;
-        const double numb = rb * inv_inc;
-        const double incb = -numb * r;
-        pb -= numb;
-        const int ee = pos ? hi_e : lo_e;
-        if (ee < 0) pb += numb;  // the extreme is the cell itself
-        else { extb = numb; ext_e = ee; }
-        gxb += incb * dd.x;
-        gyb += incb * dd.y;
-      }
-    }
+    const double numb = slope * phib * div_rn(1.0, arg_inc);
+    const double incb = -numb * r;
+    pb -= numb;
+    const int ee = arg == ps ? hi_e : lo_e;
+    if (ee < 0) pb += numb;  // the extreme is the cell itself
+    else { extb = numb; ext_e = ee; }
+    gxb += incb * dd.x;
+    gyb += incb * dd.y;
   }
   // reverse of G = sum_e coef_e (P_nb - P_c): neighbour share per entry
   for (int e = e0; e < e1; ++e) {
@@ -559,60 +558,48 @@ __device__ __forceinline__ void vjp_cell_variable(const DevGeom& g, const double
   }
 }
 
-// Resident 256-thread blocks per SM the cell reverse is compiled for.
+// Resident 64-thread blocks per SM the cell reverse is compiled for: 8 / 12 /
+// 16 give 434 / 428 / 424 us for a residual and its reverse on 131,327 cells.
 #ifndef MCFD_VJP_CELL_MIN_BLOCKS
-#define MCFD_VJP_CELL_MIN_BLOCKS 2
+#define MCFD_VJP_CELL_MIN_BLOCKS 16
 #endif
+constexpr int kCellBlock = 64;
 
+// One thread per (cell, variable).  One thread per cell held a variable's
+// state at a time in 96 registers and ran the four variables' chains one after
+// the other: 407 us per launch on the 524,288-cell O-grid, 279 us now (with the limiter taken
+// at the smallest ratio: four divisions a variable instead of eight).
 template <int LIMITER, bool FO>
-__global__ void __launch_bounds__(kBlock, MCFD_VJP_CELL_MIN_BLOCKS) k_vjp_cell(DevGeom g, const double* __restrict__ P,
-                                                     const double* __restrict__ lambda,
-                                                     const double* __restrict__ slot_bar, double ax, double ay,
-                                                     double* __restrict__ pbar, double* __restrict__ ent_bar,
-                                                     double venkat_k) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kCellBlock, MCFD_VJP_CELL_MIN_BLOCKS) k_vjp_cell(
+    DevGeom g, const double* __restrict__ P, const double* __restrict__ lambda, const double* __restrict__ slot_bar,
+    double ax, double ay, double* __restrict__ pbar, double* __restrict__ ent_bar, double venkat_k) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t >> 2, v = t & 3;
   if (i >= g.n_cells) return;
   const int c = g.cell_order[i];  // groups equal stencil sizes; outputs do not depend on the order
-  const St4 p = ld4(P + 4 * (size_t)c);
-  const double pv[4] = {p.a, p.b, p.c, p.d};
+  const double pv = P[4 * (size_t)c + v];
   const int e0 = g.grad_ptr[c], e1 = g.grad_ptr[c + 1];
   const int s0 = g.lim_ptr[c], s1 = g.lim_ptr[c + 1];
-  double pb[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int s = s0; s < s1; ++s) {
-    const St4 q = ld4(slot_bar + 4 * (size_t)g.lim_slot[s]);
-    pb[0] += q.a; pb[1] += q.b; pb[2] += q.c; pb[3] += q.d;
-  }
+  double pb = 0.0;
+  if constexpr (FO || LIMITER == MCFD_LIMITER_VENKATAKRISHNAN_K)
+    for (int s = s0; s < s1; ++s) pb += slot_bar[4 * (size_t)g.lim_slot[s] + v];
   if constexpr (!FO && LIMITER == MCFD_LIMITER_VENKATAKRISHNAN_K) {
     const double e2 = venkat_k_e2(venkat_k, g.area[c]);
-    if (s1 - s0 == 3) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable_vk<3>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar, e2);
-    } else if (s1 - s0 == 4) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable_vk<4>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar, e2);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable_vk<0>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar, e2);
-    }
+    if (s1 - s0 == 3) vjp_cell_variable_vk<3>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar, e2);
+    else if (s1 - s0 == 4) vjp_cell_variable_vk<4>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar, e2);
+    else vjp_cell_variable_vk<0>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar, e2);
   } else if (!FO) {
-    if (s1 - s0 == 3) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable<LIMITER, 3>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar);
-    } else if (s1 - s0 == 4) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable<LIMITER, 4>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) vjp_cell_variable<LIMITER, 0>(g, P, slot_bar, v, pv[v], e0, e1, s0, s1, pb[v], ent_bar);
-    }
+    if (s1 - s0 == 3) vjp_cell_variable<LIMITER, 3>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar);
+    else if (s1 - s0 == 4) vjp_cell_variable<LIMITER, 4>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar);
+    else vjp_cell_variable<LIMITER, 0>(g, P, slot_bar, v, pv, e0, e1, s0, s1, pb, ent_bar);
   }
   if (ax != 0.0 || ay != 0.0) {  // body force (solver.py:2709-2715)
-    const St4 l = ld4(lambda + 4 * (size_t)c);
-    pb[0] += l.b * ax + l.c * ay + l.d * (ax * p.b + ay * p.c);
-    pb[1] += l.d * p.a * ax;
-    pb[2] += l.d * p.a * ay;
+    const St4 l = ld4(lambda + 4 * (size_t)c), p = ld4(P + 4 * (size_t)c);
+    if (v == 0) pb += l.b * ax + l.c * ay + l.d * (ax * p.b + ay * p.c);
+    else if (v == 1) pb += l.d * p.a * ax;
+    else if (v == 2) pb += l.d * p.a * ay;
   }
-  st4(pbar + 4 * (size_t)c, St4{pb[0], pb[1], pb[2], pb[3]});
+  pbar[4 * (size_t)c + v] = pb;
 }
 
 template <bool FO>
@@ -765,17 +752,18 @@ cudaError_t launch_vjp(const DevGeom& g, const mcfd_config& cfg, const double* U
   }
   count_launch(2);
   const double ax = cfg.acceleration_x, ay = cfg.acceleration_y;
+  const int cell_blocks = (int)((4LL * C + kCellBlock - 1) / kCellBlock);
   if (fo) {
-    k_vjp_cell<0, true><<<blocks_for(C), kBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0);
+    k_vjp_cell<0, true><<<cell_blocks, kCellBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0);
     k_vjp_collect<true><<<blocks_for(C), kBlock, 0, s>>>(g, P, w.pbar, w.ent_bar, cfg.gamma, ubar);
   } else {
     switch (cfg.limiter) {
-      case 0: k_vjp_cell<0, false><<<blocks_for(C), kBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
-      case 1: k_vjp_cell<1, false><<<blocks_for(C), kBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
-      case 2: k_vjp_cell<2, false><<<blocks_for(C), kBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
-      case 3: k_vjp_cell<3, false><<<blocks_for(C), kBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
+      case 0: k_vjp_cell<0, false><<<cell_blocks, kCellBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
+      case 1: k_vjp_cell<1, false><<<cell_blocks, kCellBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
+      case 2: k_vjp_cell<2, false><<<cell_blocks, kCellBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
+      case 3: k_vjp_cell<3, false><<<cell_blocks, kCellBlock, 0, s>>>(g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, 0.0); break;
       default:
-        k_vjp_cell<MCFD_LIMITER_VENKATAKRISHNAN_K, false><<<blocks_for(C), kBlock, 0, s>>>(
+        k_vjp_cell<MCFD_LIMITER_VENKATAKRISHNAN_K, false><<<cell_blocks, kCellBlock, 0, s>>>(
             g, P, lambda, w.slot_bar, ax, ay, w.pbar, w.ent_bar, cfg.venkat_k);
         break;
     }
