@@ -172,57 +172,82 @@ __device__ __forceinline__ void gradient_sums(const DevGeom& g, const double* __
   for (; e < e1; ++e) visit(e, std::false_type{});
 }
 
-// Resident 256-thread blocks per SM the generic kernel is compiled for.
-#ifndef MCFD_RECON_GENERIC_MIN_BLOCKS
-#define MCFD_RECON_GENERIC_MIN_BLOCKS 2
-#endif
-
+// The per-face-factor reconstruction (exact variant; the smooth form in every
+// variant), one thread per (cell, variable): the variables of a cell are
+// independent, and in one thread their four chains ran one after the other.
+// Exact residual of 1,980 / 40,000 / 160,000 / 1,572,864 cells 66 / 77 / 123 /
+// 991 us with a thread per cell, 47 / 62 / 102 / 848 us so (this pass alone, on
+// 3,050 cells, 26 -> 9 us; bound by FP64 issue on the largest).
 template <int LIMITER>
-__global__ void __launch_bounds__(kBlock, MCFD_RECON_GENERIC_MIN_BLOCKS) k_reconstruct(DevGeom g, const double* __restrict__ P,
-                                                                                       double* __restrict__ recon,
-                                                                                       double venkat_k) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kBlock) k_reconstruct(DevGeom g, const double* __restrict__ P,
+                                                        double* __restrict__ recon, double venkat_k) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = t >> 2, v = t & 3;
   if (i >= g.n_cells) return;
   const int c = g.cell_order[i];
-  const St4 p = ld4(P + 4 * (size_t)c);
-  double gx[4], gy[4];
-  double lo[4] = {p.a, p.b, p.c, p.d}, hi[4] = {p.a, p.b, p.c, p.d};
-  const double pv[4] = {p.a, p.b, p.c, p.d};
-  gradient_sums(g, P, c, pv, gx, gy, lo, hi);
-  double phi[4] = {1.0, 1.0, 1.0, 1.0};
+  const double pv = P[4 * (size_t)c + v];
+  double gx = 0.0, gy = 0.0, lo = pv, hi = pv;
+  for (int e = g.grad_ptr[c], e0 = e, e1 = g.grad_ptr[c + 1]; e < e1; ++e) {
+    const double q = P[4 * (size_t)g.grad_nb[e] + v];
+    const double d = q - pv;
+    const double tx = kmul<MUL_GRADIENT>(g.grad_cx[e], d), ty = kmul<MUL_GRADIENT>(g.grad_cy[e], d);
+    if (e == e0) {  // 0.0 + t
+      gx = plus_zero(tx);
+      gy = plus_zero(ty);
+    } else {
+      gx = gx + tx;
+      gy = gy + ty;
+    }
+    if (icmp::lt(q, lo)) lo = q;
+    if (icmp::lt(hi, q)) hi = q;
+  }
+  double phi = 1.0;
   const int s0 = g.lim_ptr[c], s1 = g.lim_ptr[c + 1];
+  constexpr int kKept = 4;  // increments kept for the face values; further ones are computed again
+  double kept[kKept];
   if constexpr (LIMITER == MCFD_LIMITER_VENKATAKRISHNAN_K) {
     // minimum over the faces of the smooth face function (no cap at 1)
     const double e2 = venkat_k_e2(venkat_k, g.area[c]);
-    for (int s = s0; s < s1; ++s) {
-      const double2 d = g.lim_d[s];
+    auto visit = [&](int s, double inc) {
+      const double f = venkat_k_face(pv, inc, lo, hi, e2).f;
+      if (s == s0 || icmp::lt(f, phi)) phi = f;
+    };
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const double inc = kmul<MUL_INCREMENT>(gx[v], d.x) + kmul<MUL_INCREMENT>(gy[v], d.y);
-        const double f = venkat_k_face(pv[v], inc, lo[v], hi[v], e2).f;
-        if (s == s0 || icmp::lt(f, phi[v])) phi[v] = f;
+    for (int k = 0; k < kKept; ++k)
+      if (s0 + k < s1) {
+        const double2 r = g.lim_d[s0 + k];
+        kept[k] = kmul<MUL_INCREMENT>(gx, r.x) + kmul<MUL_INCREMENT>(gy, r.y);
+        visit(s0 + k, kept[k]);
       }
+    for (int s = s0 + kKept; s < s1; ++s) {
+      const double2 r = g.lim_d[s];
+      visit(s, kmul<MUL_INCREMENT>(gx, r.x) + kmul<MUL_INCREMENT>(gy, r.y));
     }
   } else {
-    double tol[4];
+    const double tol = limiter_tolerance(pv);
+    auto visit = [&](double inc) {
+      const double f = limiter_face_factor<LIMITER>(pv, inc, lo, hi, tol);
+      if (icmp::lt_nonneg(f, phi)) phi = f;
+    };
 #pragma unroll
-    for (int v = 0; v < 4; ++v) tol[v] = limiter_tolerance(pv[v]);
-    for (int s = s0; s < s1; ++s) {
-      const double2 d = g.lim_d[s];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        double inc = kmul<MUL_INCREMENT>(gx[v], d.x) + kmul<MUL_INCREMENT>(gy[v], d.y);
-        double f = limiter_face_factor<LIMITER>(pv[v], inc, lo[v], hi[v], tol[v]);
-        if (icmp::lt_nonneg(f, phi[v])) phi[v] = f;
+    for (int k = 0; k < kKept; ++k)
+      if (s0 + k < s1) {
+        const double2 r = g.lim_d[s0 + k];
+        kept[k] = kmul<MUL_INCREMENT>(gx, r.x) + kmul<MUL_INCREMENT>(gy, r.y);
+        visit(kept[k]);
       }
+    for (int s = s0 + kKept; s < s1; ++s) {
+      const double2 r = g.lim_d[s];
+      visit(kmul<MUL_INCREMENT>(gx, r.x) + kmul<MUL_INCREMENT>(gy, r.y));
     }
   }
-  for (int s = s0; s < s1; ++s) {
-    const double2 d = g.lim_d[s];
-    double out[4];
 #pragma unroll
-    for (int v = 0; v < 4; ++v) out[v] = pv[v] + phi[v] * (kmul<MUL_INCREMENT>(gx[v], d.x) + kmul<MUL_INCREMENT>(gy[v], d.y));
-    st4(recon + 4 * (size_t)g.lim_slot[s], St4{out[0], out[1], out[2], out[3]});
+  for (int k = 0; k < kKept; ++k)
+    if (s0 + k < s1) recon[4 * (size_t)g.lim_slot[s0 + k] + v] = pv + phi * kept[k];
+  for (int s = s0 + kKept; s < s1; ++s) {
+    const double2 r = g.lim_d[s];
+    recon[4 * (size_t)g.lim_slot[s] + v] =
+        pv + phi * (kmul<MUL_INCREMENT>(gx, r.x) + kmul<MUL_INCREMENT>(gy, r.y));
   }
 }
 
@@ -958,12 +983,13 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
                                double* recon, cudaStream_t s) {
   if (g.n_cells == 0) return cudaSuccess;
   const int t = g.tune_recon_threads ? g.tune_recon_threads : kBlock;
-  const int b = (g.n_cells + t - 1) / t;
+  const int tv = g.tune_recon_threads ? g.tune_recon_threads : 64;  // a thread per (cell, variable)
+  const int b = (int)((4LL * g.n_cells + tv - 1) / tv);
   if (cfg.limiter == MCFD_LIMITER_VENKATAKRISHNAN_K) {
     // the smooth form has no smallest-ratio shortcut: per-face evaluation in
     // every variant
     count_launch();
-    k_reconstruct<MCFD_LIMITER_VENKATAKRISHNAN_K><<<b, t, 0, s>>>(g, P, recon, cfg.venkat_k);
+    k_reconstruct<MCFD_LIMITER_VENKATAKRISHNAN_K><<<b, tv, 0, s>>>(g, P, recon, cfg.venkat_k);
     return cudaGetLastError();
   }
   if constexpr (kFast || kMinRatio) {
@@ -971,7 +997,7 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
       // 64-thread blocks by default: RK3 step of the 1024^2 vortex 2,585 us
       // against 2,591 / 2,617 with 128 / 256, of the 400^2 vortex 487 against
       // 488 / 493; smaller meshes do not tell them apart
-      const int t = g.tune_recon_threads ? g.tune_recon_threads : 64;
+      const int t = tv;
       const int bs = (int)((4LL * g.n_lim34 + t - 1) / t);
       count_launch();
       switch (cfg.limiter) {
@@ -1003,10 +1029,10 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
   } else {
     count_launch();
     switch (cfg.limiter) {
-      case 0: k_reconstruct<0><<<b, t, 0, s>>>(g, P, recon, 0.0); break;
-      case 1: k_reconstruct<1><<<b, t, 0, s>>>(g, P, recon, 0.0); break;
-      case 2: k_reconstruct<2><<<b, t, 0, s>>>(g, P, recon, 0.0); break;
-      default: k_reconstruct<3><<<b, t, 0, s>>>(g, P, recon, 0.0); break;
+      case 0: k_reconstruct<0><<<b, tv, 0, s>>>(g, P, recon, 0.0); break;
+      case 1: k_reconstruct<1><<<b, tv, 0, s>>>(g, P, recon, 0.0); break;
+      case 2: k_reconstruct<2><<<b, tv, 0, s>>>(g, P, recon, 0.0); break;
+      default: k_reconstruct<3><<<b, tv, 0, s>>>(g, P, recon, 0.0); break;
     }
   }
   return cudaGetLastError();
