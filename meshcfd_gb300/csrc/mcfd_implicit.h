@@ -187,7 +187,7 @@ struct ImplicitState {
   double* hess = nullptr;            // device [m][m + 1] Hessenberg columns
   double* givens = nullptr;          // device [3 m + 2]: c, s, S
   double* hcol = nullptr;            // device [m + 3]: dots, |w|^2 before / after
-  double* mgs_partials = nullptr;    // device [2][mgs_blocks]
+  double* mgs_partials = nullptr;    // device [3][mgs_blocks]
   int mgs_blocks = 0;
   cudaStream_t cap_stream = nullptr;  // stream the inner loop is captured on
   int inner_nodes = 0;                // nodes of one captured Arnoldi step

@@ -273,6 +273,13 @@ cudaError_t launch_bc_states(const DevGeom& g, const mcfd_config& cfg, const dou
 // summation order, so both give the same bits only while they share it.
 constexpr int kSumsqBlocks = 152 * 4;
 constexpr int kSumsqThreads = 256;
+// Blocks launched for n terms a column: those with a term.  The others of the
+// fixed grid would add +0 to non-negative sums, which changes no bit.
+// (12,200 terms: the final sum 9.5 us with all blocks, 5.1 us so.)
+inline int sumsq_blocks(long long n) {
+  const long long b = (n + kSumsqThreads - 1) / kSumsqThreads;
+  return b < 1 ? 1 : b < kSumsqBlocks ? (int)b : kSumsqBlocks;
+}
 __global__ void k_sumsq_partial(int n, const double* __restrict__ R, double* __restrict__ partials);
 __global__ void k_sumsq_final(int blocks, const double* __restrict__ partials, double* sums);
 cudaError_t finalize_time_step(DevStatus* st, double* dt_min, double time_limit, cudaStream_t s);

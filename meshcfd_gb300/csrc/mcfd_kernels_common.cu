@@ -1,6 +1,8 @@
 // Variant-independent kernels: the residual sum of squares, the launch
 // counter and the element-wise division / square root / product entry points.  Compiled
 // with -fmad=false (plain additions in a fixed tree).
+#include <algorithm>
+
 #include "mcfd_device.cuh"
 #include "mcfd_internal.h"
 #include "mcfd_reduce.cuh"
@@ -13,7 +15,8 @@ static constexpr int kBlock = 256;
 
 // Per thread a grid-stride sum, per warp a shuffle tree, per block the warps'
 // sums added in warp order by one thread: a fixed order for a fixed grid
-// (kSumsqBlocks x kSumsqThreads), so every call gives the same bits.
+// (kSumsqBlocks x kSumsqThreads, of which blocks without a cell stay away), so
+// every call gives the same bits.
 __global__ void __launch_bounds__(kSumsqThreads) k_sumsq_partial(int n, const double* __restrict__ R,
                                                                  double* __restrict__ partials) {
   __shared__ double warp_sum[kSumsqThreads / 32][4];
@@ -97,8 +100,9 @@ static long long g_launches = 0;
 long long launch_count() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
 void count_launch(int n) { __atomic_fetch_add(&g_launches, (long long)n, __ATOMIC_RELAXED); }
 
-cudaError_t launch_sumsq(const DevGeom& g, const double* R, double* partials, int blocks,
+cudaError_t launch_sumsq(const DevGeom& g, const double* R, double* partials, int max_blocks,
                          double* sums, cudaStream_t s) {
+  const int blocks = std::min(max_blocks, sumsq_blocks(g.n_cells));
   count_launch(2);
   k_sumsq_partial<<<blocks, kSumsqThreads, 0, s>>>(g.n_cells, R, partials);
   k_sumsq_final<<<1, kSumsqThreads, 0, s>>>(blocks, partials, sums);

@@ -60,9 +60,10 @@ extern "C" int mcfd_residual_sumsq_noalloc(const double* R, int64_t n_cells, dou
     scratch = g_scratch_address[device];
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int blocks = mcfd::sumsq_blocks(n_cells);
   mcfd::count_launch(2);
-  mcfd::k_sumsq_partial<<<mcfd::kSumsqBlocks, mcfd::kSumsqThreads, 0, s>>>(static_cast<int>(n_cells), R, scratch);
+  mcfd::k_sumsq_partial<<<blocks, mcfd::kSumsqThreads, 0, s>>>(static_cast<int>(n_cells), R, scratch);
   if (cudaPeekAtLastError() != cudaSuccess) return MCFD_E_CUDA;
-  mcfd::k_sumsq_final<<<1, mcfd::kSumsqThreads, 0, s>>>(mcfd::kSumsqBlocks, scratch, sums);
+  mcfd::k_sumsq_final<<<1, mcfd::kSumsqThreads, 0, s>>>(blocks, scratch, sums);
   return cudaPeekAtLastError() == cudaSuccess ? MCFD_OK : MCFD_E_CUDA;
 }
