@@ -153,10 +153,16 @@ static int ensure_viscous(mcfd_geom* h, const mcfd_config* cfg) {
   h->jvp_owned.push_back(entry);
   if (cudaMalloc((void**)&normal, 4 * C * sizeof(double)) != cudaSuccess) return MCFD_E_CUDA;
   h->jvp_owned.push_back(normal);
+  // on a stream of its own, waited for here: the caller's may be under capture
+  cudaStream_t own = nullptr;
+  if (cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) != cudaSuccess) return MCFD_E_CUDA;
+  cudaError_t e = launch_viscous_plan(h->g, entry, normal, own);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+  cudaStreamDestroy(own);
+  if (e != cudaSuccess) return MCFD_E_CUDA;
   h->g.visc_entry = entry;
   h->g.visc_normal = normal;
-  if (launch_viscous_plan(h->g, entry, normal, nullptr) != cudaSuccess) return MCFD_E_CUDA;
-  return cudaStreamSynchronize(nullptr) == cudaSuccess ? MCFD_OK : MCFD_E_CUDA;
+  return MCFD_OK;
 }
 
 static cudaError_t stage(mcfd_geom* h, const mcfd_config& cfg, const StageProgram& prog_in,

@@ -29,8 +29,8 @@
 //   quotient, store, synchronise the warp; no predicated FP64 instruction
 //   (absent entries are products of zeros) and few others, since a warp alone
 //   on its scheduler pays every instruction's latency.
-// 512 x 256 bump (131,072 cells, 767 levels of at most 256 rows): 743 us per
-// application (two sweeps, ~930 cycles a level) against 1,266 us of the
+// 512 x 256 bump (131,072 cells, 767 levels of at most 256 rows): 719 us per
+// application (two sweeps, ~900 cycles a level) against 1,266 us of the
 // windowed sweep, which bars the cluster once per window; 301 x 149 bump 433
 // against 706, 3,050 triangles 119 against 144 us.
 // The arithmetic is sweep_solve's in mcfd_implicit.cu, component by component:
