@@ -192,7 +192,8 @@ static cudaError_t stage(mcfd_geom* h, const mcfd_config& cfg, const StageProgra
   // their chain of launches runs on the side stream beside the
   // reconstruction and the fluxes, joined before the gather (both chains are
   // bound by latency on meshes that do not fill the GPU: four viscous RK2 steps
-  // on 44,849 cells 3.17 -> 2.62 ms with the gradients' plan).
+  // on 44,849 cells 3.17 -> 2.62 ms with the gradients' plan, 2.52 ms with the
+  // inlet-type faces' states ahead of the gradients).
   const bool viscous = cfg.viscosity_model != MCFD_VISC_INVISCID;
   if (viscous) {
     if (h->g.n_bc_patches > 0) e = launch_bc_states(h->g, cfg, h->ws.P, nullptr, h->g.bc_ext_dt, s);

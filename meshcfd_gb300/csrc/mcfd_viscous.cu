@@ -77,24 +77,6 @@ __device__ __forceinline__ void viscous_flux(const double g[6], double u, double
   out[3] = u * tx + v * ty + q;
 }
 
-__global__ void __launch_bounds__(kBlock) k_visc_cells(DevGeom g, const double* __restrict__ P, Visc vs,
-                                                       double* __restrict__ cell) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= g.n_cells) return;
-  const St4 p = ld4(P + 4 * (size_t)c);
-  const double T = div_rn(p.d, p.a * vs.R);
-  bool bad = false;
-  const double mu = viscosity(vs, T, &bad);
-  int bits = 0;
-  if (!isfinite(T) || !(T > 0.0)) bits |= MCFD_S_VISC_TEMPERATURE;
-  if (bad) bits |= MCFD_S_VISC_SUTHERLAND;
-  if (bits) flag(g.status, bits, c);
-  const double k = conductivity(vs, mu);
-  const double prm = vs.pr < 0.9 ? vs.pr : 0.9;
-  const double e1 = div_rn((4.0 / 3.0) * mu, p.a), e2 = div_rn(mu, p.a * prm);
-  st4(cell + 4 * (size_t)c, St4{T, mu, k, e2 > e1 ? e2 : e1});
-}
-
 // exterior (u, v, T) of an inlet-type face from the cell values
 __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, int j, int o, double2 n, double gamma,
                                              double R, double out[3], int* bits) {
@@ -110,6 +92,44 @@ __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, 
   out[1] = st.c;
   out[2] = div_rn(st.d, st.a * R);
   return true;
+}
+
+// The inlet-type faces' blocks first: their exterior states (three dependent
+// powers for a far field) take the longest, and computed here they are off the
+// gradients' and the face fluxes' chains, which both read them: (u, v, T) and
+// whether there is one, in the face's entry of bflux until its flux replaces
+// it.  44,849 cells: this launch 6.7 -> 9.1 us, the gradients 26.8 -> 15.0, the
+// face fluxes 19.1 -> 15.2.
+__global__ void __launch_bounds__(kBlock) k_visc_cells(DevGeom g, const double* __restrict__ P, Visc vs,
+                                                       double* __restrict__ cell, double* __restrict__ bflux,
+                                                       int inlet_blocks) {
+  const int b = (int)blockIdx.x;
+  if (b < inlet_blocks) {
+    const int j = b * blockDim.x + threadIdx.x;
+    if (j >= g.n_diffusive || g.diff_kind[j] != MCFD_DIFF_INLET) return;
+    const int o = g.diff_owner[j];
+    double iv[3];
+    int bits = 0;
+    const bool given = inlet_values(g, P, j, o, g.diff_normal[j], vs.gamma, vs.R, iv, &bits);
+    if (bits) flag(g.status, bits, o);
+    if (!given) iv[0] = iv[1] = iv[2] = 0.0;
+    st4(bflux + 4 * (size_t)j, St4{iv[0], iv[1], iv[2], given ? 1.0 : 0.0});
+    return;
+  }
+  const int c = (b - inlet_blocks) * blockDim.x + threadIdx.x;
+  if (c >= g.n_cells) return;
+  const St4 p = ld4(P + 4 * (size_t)c);
+  const double T = div_rn(p.d, p.a * vs.R);
+  bool bad = false;
+  const double mu = viscosity(vs, T, &bad);
+  int bits = 0;
+  if (!isfinite(T) || !(T > 0.0)) bits |= MCFD_S_VISC_TEMPERATURE;
+  if (bad) bits |= MCFD_S_VISC_SUTHERLAND;
+  if (bits) flag(g.status, bits, c);
+  const double k = conductivity(vs, mu);
+  const double prm = vs.pr < 0.9 ? vs.pr : 0.9;
+  const double e1 = div_rn((4.0 / 3.0) * mu, p.a), e2 = div_rn(mu, p.a * prm);
+  st4(cell + 4 * (size_t)c, St4{T, mu, k, e2 > e1 ? e2 : e1});
 }
 
 // The mesh-only part of the least-squares gradients, once per geometry: per
@@ -144,9 +164,11 @@ __global__ void __launch_bounds__(kBlock) k_visc_plan(DevGeom g, double2* __rest
 
 // Bound by FP64 issue and the gathers' latency; the normal matrix and the
 // weights (11 of an entry's 26 FP64 operations and its division) come from
-// the plan: 32 us per launch on 44,849 cells before, 27 us now (the boundary cells' exterior states are what is left).
-__global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const double* __restrict__ P, Visc vs,
+// the plan, the inlet-type faces' states from k_visc_cells: 32 us per launch on
+// 44,849 cells before either, 27 us with the plan, 15 us now.
+__global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const double* __restrict__ P,
                                                            const double* __restrict__ cell,
+                                                           const double* __restrict__ bflux,
                                                            double* __restrict__ grad) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= g.n_cells) return;
@@ -167,7 +189,6 @@ __global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const doub
     const double diff[3] = {q.b - cv[0], q.c - cv[1], cell[4 * (size_t)nb] - cv[2]};
     add(g.visc_entry[e], diff);
   }
-  int bits = 0;
   for (int i = g.vb_ptr[c], i1 = g.vb_ptr[c + 1]; i < i1; ++i) {
     const int j = g.vb_j[i];
     const double2 nn = g.diff_normal[j];
@@ -195,17 +216,16 @@ __global__ void __launch_bounds__(kBlock) k_visc_gradients(DevGeom g, const doub
       ghost[0] -= t * nx;
       ghost[1] -= t * ny;
     } else if (kind == MCFD_DIFF_INLET) {
-      double iv[3];
-      if (inlet_values(g, P, j, c, make_double2(nx, ny), vs.gamma, vs.R, iv, &bits)) {
-        ghost[0] = 2.0 * iv[0] - ghost[0];
-        ghost[1] = 2.0 * iv[1] - ghost[1];
-        ghost[2] = 2.0 * iv[2] - ghost[2];
+      const St4 iv = ld4(bflux + 4 * (size_t)j);
+      if (icmp::gt0(iv.d)) {
+        ghost[0] = 2.0 * iv.a - ghost[0];
+        ghost[1] = 2.0 * iv.b - ghost[1];
+        ghost[2] = 2.0 * iv.c - ghost[2];
       }
     }
     const double diff[3] = {ghost[0] - cv[0], ghost[1] - cv[1], ghost[2] - cv[2]};
     add(g.visc_entry[(size_t)g.n_gradient + j], diff);
   }
-  if (bits) flag(g.status, bits, c);
   double out[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   const St4 m = ld4(g.visc_normal + 4 * (size_t)c);
   if (icmp::gt0(m.d)) {
@@ -316,11 +336,11 @@ __device__ __forceinline__ void visc_boundary(const DevGeom& g, const double* __
     bv[0] -= nvel * nx;
     bv[1] -= nvel * ny;
   } else {
-    double iv[3];
-    if (kind == MCFD_DIFF_INLET && inlet_values(g, P, j, o, make_double2(nx, ny), vs.gamma, vs.R, iv, &bits)) {
-      bv[0] = iv[0];
-      bv[1] = iv[1];
-      bv[2] = iv[2];
+    const St4 iv = kind == MCFD_DIFF_INLET ? ld4(bflux + 4 * (size_t)j) : St4{0.0, 0.0, 0.0, 0.0};
+    if (icmp::gt0(iv.d)) {
+      bv[0] = iv.a;
+      bv[1] = iv.b;
+      bv[2] = iv.c;
 #pragma unroll
       for (int comp = 0; comp < 3; ++comp) {
         const double dn = div_rn(bv[comp] - cv[comp] - dot2(fg[2 * comp], fg[2 * comp + 1], tox, toy), nd);
@@ -444,8 +464,9 @@ cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, co
   const int t = seg_threads(C) < kBlock ? seg_threads(C) : kBlock, tf = seg_threads(nf) < kBlock ? seg_threads(nf) : kBlock;
   const int bb = (g.n_diffusive + tf - 1) / tf, fb = (nf + tf - 1) / tf;
   count_launch(4);
-  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell);
-  k_visc_gradients<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, w.grad);
+  const int ib = (g.n_diffusive + t - 1) / t;
+  k_visc_cells<<<ib + (C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, w.bflux, ib);
+  k_visc_gradients<<<(C + t - 1) / t, t, 0, s>>>(g, P, w.cell, w.bflux, w.grad);
   if (bb + fb > 0) k_visc_fluxes<<<bb + fb, tf, 0, s>>>(g, P, vs, w.cell, w.grad, w.flux, w.bflux, bb);
   k_visc_gather<<<(C + t - 1) / t, t, 0, s>>>(g, w.flux, w.bflux, w.r);
   return cudaGetLastError();
@@ -463,7 +484,7 @@ cudaError_t launch_viscous_diffusion(const DevGeom& g, const mcfd_config& cfg, c
   const int C = g.n_cells;
   const int t = seg_threads(C) < kBlock ? seg_threads(C) : kBlock;
   count_launch(2);
-  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell);
+  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, nullptr, 0);
   k_visc_diffusion<<<(C + t - 1) / t, t, 0, s>>>(g, w.cell, w.diff);
   return cudaGetLastError();
 }
