@@ -334,14 +334,14 @@ __global__ void __launch_bounds__(kBlock) k_parabolic_plan(DevGeom g, double* __
 
 // Products of the right-hand side that run on the integer pipe (mul_rn, the
 // same IEEE product): the first MCFD_PAR_INT_MUL of an entry's five.  RK3 step
-// of the 181 x 181 vortex with 0 / 1 / 2 / 3 / 5 of them: 600 / 561 / 557 /
-// 558 / 544 us; and with 8 / 10 / 11 / 12 resident 128-thread blocks: 541 /
-// 545 / 532 / 533 us.
+// of the 181 x 181 vortex with 0 / 2 / 5 of them: 478 / 437 / 396 us; and with 6
+// / 8 / 10 / 11 resident 128-thread blocks 385 / 386 / 392 / 396 us (on 36,100
+// cells 412 / 412 / 418 / 446).
 #ifndef MCFD_PAR_INT_MUL
 #define MCFD_PAR_INT_MUL 5
 #endif
 #ifndef MCFD_PAR_MIN_BLOCKS
-#define MCFD_PAR_MIN_BLOCKS 11
+#define MCFD_PAR_MIN_BLOCKS 6
 #endif
 template <int I>
 __device__ __forceinline__ double rhs_mul(double a, double b) {
@@ -349,31 +349,47 @@ __device__ __forceinline__ double rhs_mul(double a, double b) {
   else return a * b;
 }
 
-// Limiter factor and face states (or fields) of one variable for NS limiter
-// entries (NS = 0: any count, recomputing the increments).  The two sums of
-// the increment associate differently, as the reference's limiter and its
-// _reconstruct do; they share their products.
-template <int LIMITER, int NS>
+// Limiter factor and face states (or fields) of one variable, its increments
+// kept for up to four limiter entries (KEPT; else any count, recomputing the
+// increments).  The two sums of the increment associate differently, as the
+// reference's limiter and its _reconstruct do; they share their products.
+// The entries' loop stays a loop: a warp that mixes triangles and quads runs
+// each entry once (bodies compiled for 3 and for 4 entries ran one after the
+// other), and the body, some 300 instructions with its fixed-point quotients,
+// stays in the instruction cache, which warps at different places of the
+// unrolled code kept missing (7 of 24 stall cycles an issue).  FP64
+// instructions of a warp are 64 cycles apart either way, so nothing is lost by
+// the order.  RK3 step of the 181 x 181 vortex 523 us with the bodies for 3 and
+// 4 entries, 514 / 427 / 386 us unrolled by 4 / 2 / 1.
+template <int LIMITER, bool KEPT>
 __device__ __forceinline__ double parabolic_faces(const DevGeom& g, double* __restrict__ recon, int v, double pv,
                                                   int s0, int s1, double gx, double gy, double kxx, double kxy,
                                                   double kyy, double lo, double hi) {
   const double tol = limiter_tolerance(pv);
   const double hxx = 0.5 * kxx, hyy = 0.5 * kyy;
   double phi = 1.0;
-  if constexpr (NS > 0) {
-    double out[NS];
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
+  if constexpr (KEPT) {
+    const int n = s1 - s0;
+    double o0 = 0.0, o1 = 0.0, o2 = 0.0, o3 = 0.0;
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      if (k >= n) break;
       const double2 d = g.lim_d[s0 + k];
       const double t1 = gx * d.x + gy * d.y, txx = hxx * (d.x * d.x), txy = kxy * (d.x * d.y),
                    tyy = hyy * (d.y * d.y);
-      out[k] = t1 + ((txx + txy) + tyy);
+      const double out = t1 + ((txx + txy) + tyy);
       const double f = limiter_face_factor<LIMITER>(pv, ((t1 + txx) + txy) + tyy, lo, hi, tol);
       if (icmp::lt_nonneg(f, phi)) phi = f;
+      o0 = k == 0 ? out : o0;
+      o1 = k == 1 ? out : o1;
+      o2 = k == 2 ? out : o2;
+      o3 = k == 3 ? out : o3;
     }
     if (recon) {
+      const double kept[4] = {o0, o1, o2, o3};
 #pragma unroll
-      for (int k = 0; k < NS; ++k) recon[4 * (size_t)g.lim_slot[s0 + k] + v] = pv + phi * out[k];
+      for (int k = 0; k < 4; ++k)
+        if (k < n) recon[4 * (size_t)g.lim_slot[s0 + k] + v] = pv + phi * kept[k];
     }
   } else {
     for (int s = s0; s < s1; ++s) {
@@ -397,10 +413,9 @@ __device__ __forceinline__ double parabolic_faces(const DevGeom& g, double* __re
 // One thread per (cell, variable): the variables of a cell are independent
 // given the plan, and four short threads leave room for the warps that hide
 // the 64-cycle FP64 latency (the former thread per cell held 246 registers).
-// Bound by the FP64 pipe (63 % busy at 49,141 cells, where the grid is a
-// little over one wave).  RK3 step of the 181 x 181 mixed vortex: 465 us per
-// reconstruction with the plan recomputed in it, 142 us now; the step 1,372
-// against 532 us.
+// Bound by FP64 issue.  RK3 step of the 181 x 181 mixed vortex (49,141 cells):
+// 465 us per reconstruction with the plan recomputed in it, 142 us with the
+// plan, 96 us now; the step 1,372, 532 and 385 us.
 template <int LIMITER, bool FIELDS>
 __global__ void __launch_bounds__(kBlock, MCFD_PAR_MIN_BLOCKS) k_reconstruct_parabolic(DevGeom g, const double* __restrict__ P,
                                                                   double* __restrict__ recon,
@@ -465,12 +480,10 @@ __global__ void __launch_bounds__(kBlock, MCFD_PAR_MIN_BLOCKS) k_reconstruct_par
     phi = 1.0;
     if (!FIELDS)
       for (int s = s0; s < s1; ++s) recon[4 * (size_t)g.lim_slot[s] + v] = pv + 0.0;
-  } else if (s1 - s0 == 3) {
-    phi = parabolic_faces<LIMITER, 3>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
-  } else if (s1 - s0 == 4) {
-    phi = parabolic_faces<LIMITER, 4>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
+  } else if (s1 - s0 <= 4) {
+    phi = parabolic_faces<LIMITER, true>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
   } else {
-    phi = parabolic_faces<LIMITER, 0>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
+    phi = parabolic_faces<LIMITER, false>(g, out, v, pv, s0, s1, gx, gy, kxx, kxy, kyy, lo, hi);
   }
   if (FIELDS) {
     grad_out[8 * (size_t)c + 2 * v] = gx;
