@@ -52,7 +52,7 @@ def parse(argv=None):
     ap.add_argument("--no-autotune", action="store_true", help="keep the default launch shapes")
     ap.add_argument("--launch-shapes", default="",
                     help="set the stage kernels' launch shapes instead of autotuning: reconstruction threads, flux "
-                         "threads, flux faces per thread, gather threads, per-variable reconstruction (0/1), "
+                         "threads, flux faces per thread, gather threads, 0 or 1 (no effect), "
                          "e.g. 64,64,1,64,1 (mcfd_set_launch_shapes)")
     ap.add_argument("--batch-adjoint-checkpoint", type=int, default=5)
     ap.add_argument("--batch-cases", type=int, default=256)

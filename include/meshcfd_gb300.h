@@ -334,14 +334,14 @@ const double* mcfd_geom_stage_state(const mcfd_geom* geom, int32_t k);
  * reconstruction and gather threads per block in {64, 128, 256}, flux
  * threads in {64, 128, 256} x faces per thread in {1, 2, 4}.  The choice
  * stays with the handle; chosen (host [5]) receives reconstruction threads,
- * flux threads, flux faces per thread, gather threads (0: default) and
- * whether the fast variant's reconstruction runs one thread per (cell,
- * variable) (1) or per cell (0).
+ * flux threads, flux faces per thread, gather threads (0: default) and 1
+ * (the reconstruction runs one thread per (cell, variable)).
  * Synchronises the stream.  No counterpart in the reference. */
 int mcfd_autotune(mcfd_geom* geom, const mcfd_config* cfg, const double* U, int32_t* chosen, void* stream);
 /* Set the launch shapes directly (host [5], the layout mcfd_autotune fills;
- * 0 = default), e.g. to replay a tuning saved from an earlier run.  Results
- * do not depend on them.  No counterpart in the reference. */
+ * 0 = default; the fifth entry is 0 or 1, both the default), e.g. to replay a
+ * tuning saved from an earlier run.  Results do not depend on them.  No
+ * counterpart in the reference. */
 int mcfd_set_launch_shapes(mcfd_geom* geom, const int32_t* shapes);
 /* on = 1: run each explicit stage (mcfd_explicit_step, _record) as one
  * cooperative launch of one resident grid — reconstruction, face fluxes and

@@ -873,10 +873,6 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   g.dt_normal = AT(const double2*, o_dt_n);
   g.dt_len = AT(const double*, o_dt_len);
   g.dt_info = AT(const int*, o_dt_info);
-  // one thread per (cell, variable) unless a tuning says otherwise: faster at
-  // every size measured (RK3 step of the 64^2 / 400^2 / 1024^2 vortex 165 ->
-  // 110, 559 -> 488, 2,798 -> 2,585 us)
-  g.tune_recon_split = 1;
   g.status = AT(DevStatus*, o_status);
   h->status = g.status;
   h->status_next = AT(DevStatus*, o_status_next);
@@ -1033,21 +1029,15 @@ int mcfd_autotune(mcfd_geom* h, const mcfd_config* cfg, const double* U, int32_t
     else if (muscl)
       MCFD_DISPATCH(*cfg, launch_reconstruct(g, *cfg, h->ws.P, h->ws.recon, s));
   };
-  int best_recon = 0, best_flux_t = 0, best_flux_f = 1, best_gather = 0, best_split = 0;
+  int best_recon = 0, best_flux_t = 0, best_flux_f = 1, best_gather = 0;
   if (muscl) {
-    // the fast variant's reconstruction also has a kernel with one thread per
-    // (cell, variable); both give the same bits
-    const int splits = cfg->mode == MCFD_MODE_FAST && cfg->limiter != MCFD_LIMITER_VENKATAKRISHNAN_K ? 2 : 1;
     float best = 1e30f;
-    for (int sp = 0; sp < splits; ++sp)
-      for (int t : kThreads) {
-        g.tune_recon_threads = t;
-        g.tune_recon_split = sp;
-        const float ms = time_ms(recon);
-        if (ms < best) best = ms, best_recon = t, best_split = sp;
-      }
+    for (int t : kThreads) {
+      g.tune_recon_threads = t;
+      const float ms = time_ms(recon);
+      if (ms < best) best = ms, best_recon = t;
+    }
     g.tune_recon_threads = best_recon;
-    g.tune_recon_split = best_split;
   }
   recon();
   {
@@ -1079,7 +1069,7 @@ int mcfd_autotune(mcfd_geom* h, const mcfd_config* cfg, const double* U, int32_t
   chosen[1] = best_flux_t;
   chosen[2] = best_flux_f;
   chosen[3] = best_gather;
-  chosen[4] = best_split;
+  chosen[4] = 1;  // every variant takes one thread per (cell, variable)
   return rc(cudaGetLastError());
 }
 
@@ -1098,7 +1088,6 @@ int mcfd_set_launch_shapes(mcfd_geom* h, const int32_t* shapes) {
   h->g.tune_flux_threads = shapes[1];
   h->g.tune_flux_faces = shapes[2];
   h->g.tune_gather_threads = shapes[3];
-  h->g.tune_recon_split = shapes[4];
   return MCFD_OK;
 }
 

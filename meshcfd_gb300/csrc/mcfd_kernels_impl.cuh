@@ -336,89 +336,14 @@ __device__ __forceinline__ void reconstruct_cell_fast(const DevGeom& g, const do
   }
 }
 
-// The same cell for exactly NS limiter entries, one variable at a time: the
-// variable's increments, limiter factor and face values are finished before
-// the next variable starts, which keeps one variable's limiter state live
-// instead of four (fewer registers than the all-variables form, so no FP64
-// work is recomputed to relieve register pressure).  Face values are stored
-// per variable.
-template <int LIMITER, int NS>
-__device__ __forceinline__ void reconstruct_cell_fast_by_variable(const DevGeom& g, const double* __restrict__ P,
-                                                                  double* __restrict__ recon, int c,
-                                                                  const St4& p, int s0) {
-  const double pv[4] = {p.a, p.b, p.c, p.d};
-  double gx[4], gy[4];
-  double lo[4] = {p.a, p.b, p.c, p.d}, hi[4] = {p.a, p.b, p.c, p.d};
-  gradient_sums(g, P, c, pv, gx, gy, lo, hi);
-  double2 dk[NS];
-  size_t out[NS];
-#pragma unroll
-  for (int k = 0; k < NS; ++k) {
-    dk[k] = g.lim_d[s0 + k];
-    out[k] = 4 * (size_t)g.lim_slot[s0 + k];
-  }
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const double tol = limiter_tolerance(pv[v]);
-    double pos = 0.0, neg = 0.0, inc[NS];
-    bool has_pos = false, has_neg = false, flat = false;
-#pragma unroll
-    for (int k = 0; k < NS; ++k) {
-      inc[k] = kmul<MUL_INCREMENT>(gx[v], dk[k].x) + kmul<MUL_INCREMENT>(gy[v], dk[k].y);
-      if (icmp::gt_pos(inc[k], tol)) {
-        has_pos = true;
-        if (icmp::lt_nonneg(pos, inc[k])) pos = inc[k];
-      } else if (icmp::neg_gt_pos(inc[k], tol)) {
-        has_neg = true;
-        const double m = negate(inc[k]);
-        if (icmp::lt_nonneg(neg, m)) neg = m;
-      } else {
-        flat = true;
-      }
-    }
-    double phi;
-    if constexpr (kMinRatio)
-      phi = limiter_factor_min_ratio<LIMITER>(pv[v], lo[v], hi[v], pos, negate(neg), has_pos, has_neg, flat);
-    else
-      phi = limiter_factor_fast<LIMITER>(hi[v] - pv[v], pos, pv[v] - lo[v], neg, has_pos, has_neg, flat);
-#pragma unroll
-    for (int k = 0; k < NS; ++k) recon[out[k] + v] = pv[v] + kmul<MUL_OUTPUT>(phi, inc[k]);
-  }
-}
-
-// Register bound of the 3 / 4-entry kernel: MCFD_RECON_MAXNREG caps the
-// registers a thread directly; otherwise the bound is MCFD_RECON_MIN_BLOCKS
-// resident 256-thread blocks per SM.
-#ifndef MCFD_RECON_MIN_BLOCKS
-#define MCFD_RECON_MIN_BLOCKS 3
-#endif
-#ifdef MCFD_RECON_MAXNREG
-#define MCFD_RECON_BOUND __maxnreg__(MCFD_RECON_MAXNREG)
-#else
-#define MCFD_RECON_BOUND __launch_bounds__(kBlock, MCFD_RECON_MIN_BLOCKS)
-#endif
-
-// Cells with 3 or 4 limiter entries (cell_order[0 .. n_lim34)); the kernel
-// for any other count is separate, so that its register budget does not set
-// this one's occupancy.
-template <int LIMITER>
-__global__ void MCFD_RECON_BOUND k_reconstruct_fast(DevGeom g, const double* __restrict__ P, double* __restrict__ recon) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.n_lim34) return;
-  const int c = g.cell_order[i];
-  const St4 p = ld4(P + 4 * (size_t)c);
-  const int s0 = g.lim_ptr[c];
-  if (g.lim_ptr[c + 1] - s0 == 3) reconstruct_cell_fast_by_variable<LIMITER, 3>(g, P, recon, c, p, s0);
-  else reconstruct_cell_fast_by_variable<LIMITER, 4>(g, P, recon, c, p, s0);
-}
-
-// The same reconstruction with one thread per (cell, variable): the four
-// variables of a cell are independent (gradient, extremes, limiter and face
-// values of variable v read only variable v), so four adjacent threads take
-// one cell's variables and run exactly the per-variable code above, with a
-// quarter of its registers: more warps per SM to hide the latency of the
-// integer-pipe divisions.  Cells with 3 or 4 limiter entries; results are
-// those of k_reconstruct_fast.
+// The same reconstruction with one thread per (cell, variable), for exactly NS
+// limiter entries: the four variables of a cell are independent (gradient,
+// extremes, limiter and face values of variable v read only variable v), so
+// four adjacent threads take one cell's variables, with a quarter of a
+// cell's registers: more warps per SM to hide the latency of the integer-pipe
+// divisions.  Cells with 3 or 4 limiter entries (cell_order[0 .. n_lim34)).  A
+// thread per cell was slower at every size: RK3 step of the 64^2 / 400^2 /
+// 1024^2 vortex 165 against 110, 559 against 488, 2,798 against 2,585 us.
 template <int LIMITER, int NS>
 __device__ __forceinline__ void reconstruct_variable_fast(const DevGeom& g, const double* __restrict__ P,
                                                           double* __restrict__ recon, int c, int v, double pv,
@@ -982,7 +907,6 @@ cudaError_t launch_primitive(const DevGeom& g, const mcfd_config& cfg, const dou
 cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const double* P,
                                double* recon, cudaStream_t s) {
   if (g.n_cells == 0) return cudaSuccess;
-  const int t = g.tune_recon_threads ? g.tune_recon_threads : kBlock;
   const int tv = g.tune_recon_threads ? g.tune_recon_threads : 64;  // a thread per (cell, variable)
   const int b = (int)((4LL * g.n_cells + tv - 1) / tv);
   if (cfg.limiter == MCFD_LIMITER_VENKATAKRISHNAN_K) {
@@ -993,27 +917,17 @@ cudaError_t launch_reconstruct(const DevGeom& g, const mcfd_config& cfg, const d
     return cudaGetLastError();
   }
   if constexpr (kFast || kMinRatio) {
-    if (g.n_lim34 > 0 && g.tune_recon_split) {
+    if (g.n_lim34 > 0) {
       // 64-thread blocks by default: RK3 step of the 1024^2 vortex 2,585 us
       // against 2,591 / 2,617 with 128 / 256, of the 400^2 vortex 487 against
       // 488 / 493; smaller meshes do not tell them apart
-      const int t = tv;
-      const int bs = (int)((4LL * g.n_lim34 + t - 1) / t);
+      const int bs = (int)((4LL * g.n_lim34 + tv - 1) / tv);
       count_launch();
       switch (cfg.limiter) {
-        case 0: k_reconstruct_fast_split<0><<<bs, t, 0, s>>>(g, P, recon); break;
-        case 1: k_reconstruct_fast_split<1><<<bs, t, 0, s>>>(g, P, recon); break;
-        case 2: k_reconstruct_fast_split<2><<<bs, t, 0, s>>>(g, P, recon); break;
-        default: k_reconstruct_fast_split<3><<<bs, t, 0, s>>>(g, P, recon); break;
-      }
-    } else if (g.n_lim34 > 0) {
-      const int b34 = (g.n_lim34 + t - 1) / t;
-      count_launch();
-      switch (cfg.limiter) {
-        case 0: k_reconstruct_fast<0><<<b34, t, 0, s>>>(g, P, recon); break;
-        case 1: k_reconstruct_fast<1><<<b34, t, 0, s>>>(g, P, recon); break;
-        case 2: k_reconstruct_fast<2><<<b34, t, 0, s>>>(g, P, recon); break;
-        default: k_reconstruct_fast<3><<<b34, t, 0, s>>>(g, P, recon); break;
+        case 0: k_reconstruct_fast_split<0><<<bs, tv, 0, s>>>(g, P, recon); break;
+        case 1: k_reconstruct_fast_split<1><<<bs, tv, 0, s>>>(g, P, recon); break;
+        case 2: k_reconstruct_fast_split<2><<<bs, tv, 0, s>>>(g, P, recon); break;
+        default: k_reconstruct_fast_split<3><<<bs, tv, 0, s>>>(g, P, recon); break;
       }
     }
     if (g.n_cells > g.n_lim34) {
