@@ -332,7 +332,10 @@ const double* mcfd_geom_stage_state(const mcfd_geom* geom, int32_t k);
 /* Choose the launch shapes of the stage kernels for this geometry and
  * settings by timing candidates on the state U (device [n_cells][4]):
  * reconstruction and gather threads per block in {64, 128, 256}, flux
- * threads in {64, 128, 256} x faces per thread in {1, 2, 4}.  The choice
+ * threads in {64, 128, 256} x faces per thread in {1, 2, 4}.  Up to 500,000
+ * faces one launch takes every face segment at one face a thread; more faces
+ * a thread launch each segment by itself.  A flux shape applies to launches of
+ * at least 152 x its threads faces.  The choice
  * stays with the handle; chosen (host [5]) receives reconstruction threads,
  * flux threads, flux faces per thread, gather threads (0: default) and 1
  * (the reconstruction runs one thread per (cell, variable)).

@@ -1046,7 +1046,7 @@ int mcfd_autotune(mcfd_geom* h, const mcfd_config* cfg, const double* U, int32_t
       for (int f : kFaces) {
         g.tune_flux_threads = t;
         g.tune_flux_faces = f;
-        const float ms = time_ms([&] { MCFD_DISPATCH(*cfg, launch_flux(g, *cfg, h->ws.P, h->ws.recon, h->ws.flux, s, nullptr)); });
+        const float ms = time_ms([&] { MCFD_DISPATCH(*cfg, launch_flux(g, *cfg, h->ws.P, h->ws.recon, h->ws.flux, s, &h->side)); });
         if (ms < best) best = ms, best_flux_t = t, best_flux_f = f;
       }
     g.tune_flux_threads = best_flux_t;

@@ -221,14 +221,13 @@ inline int seg_blocks(int n) { return (n + seg_threads(n) - 1) / seg_threads(n);
 #define MCFD_MERGED_FLUX_FACES 500000
 #endif
 constexpr int kMergedFluxFaces = MCFD_MERGED_FLUX_FACES;
-// flux launch shape with the autotuned threads / faces per thread, if any
-inline int flux_threads(const DevGeom& g, int n) {
-  return g.tune_flux_threads && n >= 152 * g.tune_flux_threads ? g.tune_flux_threads : seg_threads(n);
-}
+// Flux launch shape of n faces with the tuned threads and faces per thread,
+// if any; a shape that would leave SMs without a block is not taken.
+inline bool flux_tuned(const DevGeom& g, int n) { return g.tune_flux_threads && n >= 152 * g.tune_flux_threads; }
+inline int flux_threads(const DevGeom& g, int n) { return flux_tuned(g, n) ? g.tune_flux_threads : seg_threads(n); }
+inline int flux_faces(const DevGeom& g, int n) { return flux_tuned(g, n) && g.tune_flux_faces > 1 ? g.tune_flux_faces : 1; }
 inline int flux_blocks(const DevGeom& g, int n) {
-  const int t = flux_threads(g, n);
-  const int per_block = t * (g.tune_flux_threads && n >= 152 * g.tune_flux_threads && g.tune_flux_faces > 1
-                                 ? g.tune_flux_faces : 1);
+  const int per_block = flux_threads(g, n) * flux_faces(g, n);
   return (n + per_block - 1) / per_block;
 }
 

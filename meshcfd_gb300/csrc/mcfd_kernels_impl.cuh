@@ -959,8 +959,9 @@ template <int FLUX, bool FO, bool KH>
 static void flux_segments(const DevGeom& g, const double* P, const double* recon, double* flux,
                           double gamma, cudaStream_t s, const SideStream* side) {
   const double inv_gm1 = 1.0 / (gamma - 1.0);
-  if (g.n_flux > 0 && g.n_flux <= kMergedFluxFaces) {
-    const int t = seg_threads(g.n_flux);
+  // one launch takes a tuned block size, a launch per segment tuned faces per thread
+  if (g.n_flux > 0 && g.n_flux <= kMergedFluxFaces && flux_faces(g, g.seg_begin[SEG_INTERIOR + 1]) == 1) {
+    const int t = flux_threads(g, g.n_flux);
     int blocks = 0;
     for (int k = 0; k < SEG_COUNT; ++k) blocks += (g.seg_begin[k + 1] - g.seg_begin[k] + t - 1) / t;
     count_launch();
