@@ -38,8 +38,14 @@
 // solution times the clamped diagonal straight into the backward sweep's
 // staged right-hand sides.
 //
-// Every wait is bounded: one that runs out sets MCFD_S_SWEEP_TIMEOUT and the
-// thread stops waiting; all blocks still reach the closing cluster barrier,
+// Every wait is bounded by a number of polls, enough for the longest plan (a
+// one-cell-wide strip, whose bands run one after another).  One that runs out
+// sets MCFD_S_SWEEP_TIMEOUT and ends its warp's waiting: a solver goes on with
+// whatever is there, a publisher stores and pushes nothing any more.  What a
+// warp may then still touch is in bounds: the staged rows' slots start as
+// zeros and are only ever replaced by the plan's, a chunk is copied only when
+// the one before it in its place has landed, and the copying warp waits for
+// the copies that it issued.  All blocks reach the closing cluster barrier,
 // which keeps each block's shared memory alive until the last push arrived.
 #include <cooperative_groups.h>
 
@@ -72,7 +78,16 @@ constexpr int kStagedRows = kStages * kPipeChunk;
 constexpr int F_DIAG = 0, F_VAL01 = 1024, F_VAL23 = 2048, F_META = 3072, F_RHS = 4096, F_CLAMP = 6144;
 constexpr int kChunkBytes = 6656, kChunkDoubles = kChunkBytes / 8;
 constexpr unsigned kEmptyHi = 0x7ff4a5a5u;  // high word of a signalling NaN: no arithmetic result
-constexpr int kSpinLimit = 1 << 22;
+// Polls a wait may take: one that may have to outlast the steps of all other
+// bands in sequence, of the longest plan (a step takes up to 1,050 cycles and a
+// poll at least 20, so 128 polls a step cover it more than twice; 16.5 M polls
+// of some 100 cycles pass in a second), and one for a copy to land.
+// Compile-time: as a launch argument the limit made the waiting loops 2 % of
+// the small meshes' sweeps slower.
+#ifndef MCFD_PIPELINE_SPINS
+#define MCFD_PIPELINE_SPINS (16 * kMaxSteps * 128 + (1 << 22))
+#endif
+constexpr int kSpins = MCFD_PIPELINE_SPINS, kCopySpins = 1 << 22;
 // a step's word: first row, rows - 1, then flags
 constexpr unsigned W_MANY = 1u << 29;  // rows of more than two entries
 constexpr unsigned W_WAIT = 1u << 30;  // its last row opens a chunk
@@ -113,8 +128,8 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
-  for (int i = 0; i < kSpinLimit; ++i)
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, int spins) {
+  for (int i = 0; i < spins; ++i)
     if (mbar_try(bar, parity)) return true;
   return false;
 }
@@ -210,6 +225,9 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
     reinterpret_cast<unsigned long long*>(sl)[(size_t)pair * kSlots * 2 + 2 * kRing + e] = (unsigned long long)kEmptyHi << 32;
   }
   if (t < 4) sl[(size_t)(t & 1) * kSlots * 2 + 2 * kZeroSlot + (t >> 1)] = 0.0;
+  if (warp == 2 * GROUPS + 2)
+    for (int i = lane; i < kStagedRows; i += 32)
+      reinterpret_cast<uint4*>(smem + kOffStage + kStages * F_META)[i] = make_uint4(0u, 0u, 0u, 0u);
   for (int i = t; i < n_steps; i += nt) steps[i] = a.steps[a.step0[band] + i];
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -220,7 +238,7 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
   int ready = 0, freed = 0;
   auto chunks_of = [&](unsigned w) {
     if (w & W_WAIT) {
-      if (!dead) dead = !mbar_wait(bars + 8 * (ready % kStages), (ready / kStages) & 1);
+      if (!dead) dead = !mbar_wait(bars + 8 * (ready % kStages), (ready / kStages) & 1, kSpins);
       ++ready;
     }
     if (w & W_FREE) {
@@ -233,9 +251,12 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
     // ---- the copies, kStages chunks ahead, one per field of a chunk
     if (lane == 0) {
       const unsigned char* src = reinterpret_cast<const unsigned char*>(a.stage) + (size_t)a.chunk0[band] * kChunkBytes;
-      for (int c = 0; c < n_chunks; ++c, src += kChunkBytes) {
-        const int s = c % kStages, use = c / kStages;
-        if (use > 0) dead = !mbar_wait(bars + 8 * (kStages + s), (use - 1) & 1);
+      int issued = 0;
+      for (; issued < n_chunks; ++issued, src += kChunkBytes) {
+        const int s = issued % kStages, use = issued / kStages;
+        if (use > 0)  // handed back, and landed (a warp that stopped waiting hands back early)
+          dead = !mbar_wait(bars + 8 * (kStages + s), (use - 1) & 1, kSpins) ||
+                 !mbar_wait(bars + 8 * s, (use - 1) & 1, kCopySpins);
         if (dead) break;  // the solvers' own waits run out too
         mbar_expect(bars + 8 * s, kChunkBytes);
 #pragma unroll
@@ -244,9 +265,8 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
         bulk_load(stage + kStages * F_CLAMP + 512 * s, src + F_CLAMP, 512, bars + 8 * s);
       }
       // no copy may be in flight when the block ends
-      if (!dead)
-        for (int c = n_chunks > kStages ? n_chunks - kStages : 0; c < n_chunks; ++c)
-          mbar_wait(bars + 8 * (c % kStages), (c / kStages) & 1);
+      for (int c = issued > kStages ? issued - kStages : 0; c < issued; ++c)
+        if (!mbar_wait(bars + 8 * (c % kStages), (c / kStages) & 1, kCopySpins)) dead = true;
     }
   } else if (warp >= 2 * GROUPS) {
     // ---- publishing: the solved rows of each step, behind the solvers
@@ -261,10 +281,11 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
           int done;
           asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];" : "=r"(done) : "r"(progress + 4u * (2 * g + pair)) : "memory");
           if (done > s) break;
-          if (++spins > kSpinLimit) dead = true;
+          if (++spins > kSpins) dead = true;
         }
       }
-      __syncwarp();
+      dead = __any_sync(0xffffffffu, dead);
+      if (dead) break;
 #pragma unroll
       for (int g = 0; g < GROUPS; ++g) {
         const int k = 16 * g + (lane & 15);
@@ -341,7 +362,7 @@ __global__ void __launch_bounds__(32 * (2 * GROUPS + 3), 1) k_lusgs_pipeline(Pip
         // this warp's own last step, so that is announced first
         announce(s);
         for (int spins = 0; __any_sync(0xffffffffu, empty(x0) | empty(x1) | empty(x2) | empty(x3)); ++spins) {
-          if (dead || spins > kSpinLimit) {
+          if (__any_sync(0xffffffffu, dead) || spins > kSpins) {  // the lanes leave together
             dead = true;
             break;
           }
