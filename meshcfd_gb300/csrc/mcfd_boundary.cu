@@ -18,7 +18,7 @@
 //   normal velocity from the patch flow rate, tangential velocity kept.
 // Checks set the reference's error bits and the lowest failing patch index.
 // Python's scalar x**2 is libm pow and NumPy's array power its own SIMD code;
-// both are reproduced only to the last place (x * x and CUDA pow here).
+// both are reproduced only to the last place (x * x and mode_pow here).
 #include "mcfd_device.cuh"
 #include "mcfd_internal.h"
 
@@ -130,6 +130,7 @@ __device__ __forceinline__ double invariant_at(double m, double dn, double a0, d
   return sound * (dn * m + div_rn(2.0, gamma - 1.0));
 }
 
+template <bool LIBRARY>
 __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* recon, double gamma, double R,
                                int patch, double* ext) {
   const int base = g.seg_begin[SEG_BCX];
@@ -184,7 +185,7 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
       }
       const double m = 0.5 * (low + high);
       const double t = div_rn(tt, 1.0 + 0.5 * (gamma - 1.0) * (m * m));
-      const double p = pt * pow_rn(div_rn(t, tt), div_rn(gamma, gamma - 1.0));
+      const double p = pt * mode_pow<LIBRARY>(div_rn(t, tt), div_rn(gamma, gamma - 1.0));
       const double rho = div_rn(p, R * t);
       const double speed = m * sqrt_rn(gamma * R * t);
       out = St4{rho, speed * dx, speed * dy, p};
@@ -330,12 +331,13 @@ __device__ void mass_flow_outlet(const DevGeom& g, const double* P, const double
   }
 }
 
+template <bool LIBRARY>
 __global__ void __launch_bounds__(kBlock) k_bc_states(DevGeom g, const double* __restrict__ P,
                                                       const double* __restrict__ recon, double gamma, double R,
                                                       double* __restrict__ ext) {
   const int patch = blockIdx.x;
   const int kind = g.bc_kind[patch];
-  if (kind == MCFD_BC_PRESSURE_INLET) pressure_inlet(g, P, recon, gamma, R, patch, ext);
+  if (kind == MCFD_BC_PRESSURE_INLET) pressure_inlet<LIBRARY>(g, P, recon, gamma, R, patch, ext);
   else if (kind == MCFD_BC_MASS_FLOW_OUTLET) mass_flow_outlet(g, P, recon, patch, ext);
   else if (blockIdx.y == 0) mass_flow_inlet(g, P, recon, gamma, R, patch, ext);
 }
@@ -350,7 +352,10 @@ cudaError_t launch_bc_states(const DevGeom& g, const mcfd_config& cfg, const dou
   const int faces = g.seg_begin[SEG_BCX + 1] - g.seg_begin[SEG_BCX];
   const int split = (faces + kBlock - 1) / kBlock;
   const dim3 grid(g.n_bc_patches, split < 1 ? 1 : split > 64 ? 64 : split);
-  k_bc_states<<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
+  if (cfg.mode == MCFD_MODE_EXACT)
+    k_bc_states<true><<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
+  else
+    k_bc_states<false><<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
   return cudaGetLastError();
 }
 

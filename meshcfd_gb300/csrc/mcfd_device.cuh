@@ -283,19 +283,21 @@ __device__ __forceinline__ int roe_flux(const St4& L, const St4& R, double nx, d
   return 0;
 }
 
-// The far-field state's power.  The exact variant keeps the CUDA library's:
-// it is the implicit path's default, whose finite-difference products divide
-// a residual's last places by 1.5e-8, so that another power, however close,
-// moves its linear solutions by some 1e-9 (measured 1.1e-9 on the 512 x 256
-// bump).  Every other unit takes the fixed-point one.
-#ifdef MCFD_LIBRARY_POW
-__device__ __forceinline__ double far_pow(double x, double y) { return pow(x, y); }
-#else
-__device__ __forceinline__ double far_pow(double x, double y) { return pow_rn(x, y); }
-#endif
+// The power of a boundary state or of a viscosity.  Exact mode (LIBRARY) keeps
+// the CUDA library's, in every unit: it is the implicit path's default, whose
+// finite-difference products divide a residual's last places by 1.5e-8, so
+// that another power, however close, moves its linear solutions by some 1e-9
+// (measured 1.1e-9 on the 512 x 256 bump).  The other modes take the
+// fixed-point one.
+template <bool LIBRARY>
+__device__ __forceinline__ double mode_pow(double x, double y) {
+  if constexpr (LIBRARY) return pow(x, y);
+  else return pow_rn(x, y);
+}
 
 // Far-field characteristic ghost state (solver.py:4350-4409), one face.
 // Returns a status bit (0 if fine).
+template <bool LIBRARY>
 __device__ __forceinline__ int far_field_state(const St4& in, const St4& far, double nx,
                                                double ny, double gamma, St4* ext) {
   double un_i = in.b * nx + in.c * ny;
@@ -319,9 +321,9 @@ __device__ __forceinline__ int far_field_state(const St4& in, const St4& far, do
     return MCFD_S_FARFIELD_SOUND;
   }
   const St4& src = icmp::ge0(vb) ? in : far;
-  double entropy = div_rn(src.d, far_pow(src.a, gamma));
-  double rho = far_pow(div_rn(cb * cb, gamma * entropy), div_rn(1.0, gamma - 1.0));
-  double p = entropy * far_pow(rho, gamma);
+  double entropy = div_rn(src.d, mode_pow<LIBRARY>(src.a, gamma));
+  double rho = mode_pow<LIBRARY>(div_rn(cb * cb, gamma * entropy), div_rn(1.0, gamma - 1.0));
+  double p = entropy * mode_pow<LIBRARY>(rho, gamma);
   double tx = -ny, ty = nx;
   double vt = src.b * tx + src.c * ty;
   St4 s{rho, vb * nx + vt * tx, vb * ny + vt * ty, p};

@@ -35,10 +35,6 @@
 #define MCFD_FLUX_INT_MUL 4
 #endif
 
-#if MCFD_FAST == 0
-#define MCFD_LIBRARY_POW  // far_pow (mcfd_device.cuh)
-#endif
-
 #include <cooperative_groups.h>
 
 #include <type_traits>
@@ -54,6 +50,7 @@ namespace cg = cooperative_groups;
 static constexpr int kBlock = 256;
 static constexpr bool kFast = MCFD_FAST == 2;      // fast arithmetic (fluxes, primitive)
 static constexpr bool kMinRatio = MCFD_FAST == 1;  // min-ratio limiter, exact arithmetic
+static constexpr bool kLibraryPow = MCFD_FAST == 0;  // mode_pow
 
 // Products that the exact-arithmetic variants evaluate on the integer pipe
 // (mul_rn, the same IEEE result) to take load off the FP64 pipe, which bounds
@@ -470,7 +467,7 @@ __device__ __forceinline__ void flux_face(const DevGeom& g, const double* P, con
   } else if (SEG == SEG_POUT) {
     R = St4{L.a, L.b, L.c, g.ff_pout_pressure[f - begin]};  // solver.py:2581-2582
   } else if (SEG == SEG_FAR) {
-    bits |= far_field_state(L, ld4(g.ff_far_state + 4 * (size_t)(f - begin)), n.x, n.y, gamma, &R);
+    bits |= far_field_state<kLibraryPow>(L, ld4(g.ff_far_state + 4 * (size_t)(f - begin)), n.x, n.y, gamma, &R);
   } else {
     R = ld4(g.bc_ext + 4 * (size_t)(f - begin));  // solver.py:2626-2698, states from k_bc_states
   }
@@ -562,7 +559,7 @@ __device__ __forceinline__ double far_radius(const St4& in, const St4& far, doub
     }
   }
   St4 ext;
-  *bits |= far_field_state(in, far, nx, ny, gamma, &ext);
+  *bits |= far_field_state<kLibraryPow>(in, far, nx, ny, gamma, &ext);
   return abs_of(ext.b * nx + ext.c * ny) + sound_speed(ext.a, ext.d, gamma);
 }
 

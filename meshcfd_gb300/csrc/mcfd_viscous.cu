@@ -22,7 +22,7 @@
 // fma(a1, b1, a0 * b0); a k x 2 matrix times a 2-vector (k >= 2) is its gemv,
 // fma(a0, b0, a1 * b1) per row: written out here, so constant-viscosity cases
 // follow the reference's rounding.  Sutherland's (T / Tref)^1.5 is NumPy's
-// array power there and CUDA pow here (last-place differences).
+// array power there and mode_pow here (last-place differences).
 #include "mcfd_device.cuh"
 #include "mcfd_internal.h"
 
@@ -49,9 +49,10 @@ struct Visc {
 };
 
 // _dynamic_viscosity; *bad set when Sutherland's law gives an invalid value
+template <bool LIBRARY>
 __device__ __forceinline__ double viscosity(const Visc& v, double T, bool* bad) {
   if (v.model == MCFD_VISC_CONSTANT) return v.mu0;
-  double mu = v.suth_mu * pow_rn(div_rn(T, v.suth_t), 1.5);
+  double mu = v.suth_mu * mode_pow<LIBRARY>(div_rn(T, v.suth_t), 1.5);
   mu *= div_rn(v.suth_t + v.suth_s, T + v.suth_s);
   if (!isfinite(mu) || !(mu > 0.0)) *bad = true;
   return mu;
@@ -78,6 +79,7 @@ __device__ __forceinline__ void viscous_flux(const double g[6], double u, double
 }
 
 // exterior (u, v, T) of an inlet-type face from the cell values
+template <bool LIBRARY>
 __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, int j, int o, double2 n, double gamma,
                                              double R, double out[3], int* bits) {
   const int code = g.diff_inlet[j];
@@ -85,7 +87,7 @@ __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, 
   St4 st;
   if (src == 1) st = ld4(g.ff_vin_state + 4 * (size_t)idx);
   else if (src == 2) st = ld4(g.bc_ext_dt + 4 * (size_t)idx);
-  else if (src == 3) *bits |= far_field_state(ld4(P + 4 * (size_t)o), ld4(g.ff_far_state + 4 * (size_t)idx), n.x, n.y,
+  else if (src == 3) *bits |= far_field_state<LIBRARY>(ld4(P + 4 * (size_t)o), ld4(g.ff_far_state + 4 * (size_t)idx), n.x, n.y,
                                               gamma, &st);
   else return false;
   out[0] = st.b;
@@ -100,6 +102,7 @@ __device__ __forceinline__ bool inlet_values(const DevGeom& g, const double* P, 
 // whether there is one, in the face's entry of bflux until its flux replaces
 // it.  44,849 cells: this launch 6.7 -> 9.1 us, the gradients 26.8 -> 15.0, the
 // face fluxes 19.1 -> 15.2.
+template <bool LIBRARY>
 __global__ void __launch_bounds__(kBlock) k_visc_cells(DevGeom g, const double* __restrict__ P, Visc vs,
                                                        double* __restrict__ cell, double* __restrict__ bflux,
                                                        int inlet_blocks) {
@@ -110,7 +113,7 @@ __global__ void __launch_bounds__(kBlock) k_visc_cells(DevGeom g, const double* 
     const int o = g.diff_owner[j];
     double iv[3];
     int bits = 0;
-    const bool given = inlet_values(g, P, j, o, g.diff_normal[j], vs.gamma, vs.R, iv, &bits);
+    const bool given = inlet_values<LIBRARY>(g, P, j, o, g.diff_normal[j], vs.gamma, vs.R, iv, &bits);
     if (bits) flag(g.status, bits, o);
     if (!given) iv[0] = iv[1] = iv[2] = 0.0;
     st4(bflux + 4 * (size_t)j, St4{iv[0], iv[1], iv[2], given ? 1.0 : 0.0});
@@ -121,7 +124,7 @@ __global__ void __launch_bounds__(kBlock) k_visc_cells(DevGeom g, const double* 
   const St4 p = ld4(P + 4 * (size_t)c);
   const double T = div_rn(p.d, p.a * vs.R);
   bool bad = false;
-  const double mu = viscosity(vs, T, &bad);
+  const double mu = viscosity<LIBRARY>(vs, T, &bad);
   int bits = 0;
   if (!isfinite(T) || !(T > 0.0)) bits |= MCFD_S_VISC_TEMPERATURE;
   if (bad) bits |= MCFD_S_VISC_SUTHERLAND;
@@ -262,6 +265,7 @@ __device__ __forceinline__ void visc_face(const DevGeom& g, const double* __rest
   st4(flux + 4 * (size_t)i, St4{out[0], out[1], out[2], out[3]});
 }
 
+template <bool LIBRARY>
 __device__ __forceinline__ void visc_boundary(const DevGeom& g, const double* __restrict__ P, const Visc& vs,
                                               const double* __restrict__ cell, const double* __restrict__ grad,
                                               double* __restrict__ bflux, int j) {
@@ -360,7 +364,7 @@ __device__ __forceinline__ void visc_boundary(const DevGeom& g, const double* __
     }
   }
   bool bad = false;
-  const double mu = viscosity(vs, bv[2], &bad);
+  const double mu = viscosity<LIBRARY>(vs, bv[2], &bad);
   if (bad) bits |= MCFD_S_VISC_SUTHERLAND;
   const double k = conductivity(vs, mu);
   double out[4];
@@ -374,6 +378,7 @@ __device__ __forceinline__ void visc_boundary(const DevGeom& g, const double* __
 // The face fluxes: the diffusive boundary faces' blocks first (their chain of
 // divisions and Sutherland's power is the longest), then interior and
 // periodic faces.
+template <bool LIBRARY>
 __global__ void __launch_bounds__(kBlock) k_visc_fluxes(DevGeom g, const double* __restrict__ P, Visc vs,
                                                         const double* __restrict__ cell,
                                                         const double* __restrict__ grad, double* __restrict__ flux,
@@ -381,7 +386,7 @@ __global__ void __launch_bounds__(kBlock) k_visc_fluxes(DevGeom g, const double*
   const int b = (int)blockIdx.x;
   if (b < boundary_blocks) {
     const int j = b * blockDim.x + threadIdx.x;
-    if (j < g.n_diffusive) visc_boundary(g, P, vs, cell, grad, bflux, j);
+    if (j < g.n_diffusive) visc_boundary<LIBRARY>(g, P, vs, cell, grad, bflux, j);
   } else {
     const int i = (b - boundary_blocks) * blockDim.x + threadIdx.x;
     if (i < g.seg_begin[SEG_PERIODIC + 1]) visc_face(g, P, cell, grad, flux, i);
@@ -457,7 +462,8 @@ Visc visc_of(const mcfd_config& cfg) {
 
 }  // namespace
 
-cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, const double* P, const ViscousWork& w,
+template <bool LIBRARY>
+static cudaError_t viscous_residual(const DevGeom& g, const mcfd_config& cfg, const double* P, const ViscousWork& w,
                                     cudaStream_t s) {
   const Visc vs = visc_of(cfg);
   const int C = g.n_cells, nf = g.seg_begin[SEG_PERIODIC + 1];
@@ -465,11 +471,16 @@ cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, co
   const int bb = (g.n_diffusive + tf - 1) / tf, fb = (nf + tf - 1) / tf;
   count_launch(4);
   const int ib = (g.n_diffusive + t - 1) / t;
-  k_visc_cells<<<ib + (C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, w.bflux, ib);
+  k_visc_cells<LIBRARY><<<ib + (C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, w.bflux, ib);
   k_visc_gradients<<<(C + t - 1) / t, t, 0, s>>>(g, P, w.cell, w.bflux, w.grad);
-  if (bb + fb > 0) k_visc_fluxes<<<bb + fb, tf, 0, s>>>(g, P, vs, w.cell, w.grad, w.flux, w.bflux, bb);
+  if (bb + fb > 0) k_visc_fluxes<LIBRARY><<<bb + fb, tf, 0, s>>>(g, P, vs, w.cell, w.grad, w.flux, w.bflux, bb);
   k_visc_gather<<<(C + t - 1) / t, t, 0, s>>>(g, w.flux, w.bflux, w.r);
   return cudaGetLastError();
+}
+
+cudaError_t launch_viscous_residual(const DevGeom& g, const mcfd_config& cfg, const double* P, const ViscousWork& w,
+                                    cudaStream_t s) {
+  return cfg.mode == MCFD_MODE_EXACT ? viscous_residual<true>(g, cfg, P, w, s) : viscous_residual<false>(g, cfg, P, w, s);
 }
 
 cudaError_t launch_viscous_plan(const DevGeom& g, double2* entry, double* normal, cudaStream_t s) {
@@ -484,7 +495,8 @@ cudaError_t launch_viscous_diffusion(const DevGeom& g, const mcfd_config& cfg, c
   const int C = g.n_cells;
   const int t = seg_threads(C) < kBlock ? seg_threads(C) : kBlock;
   count_launch(2);
-  k_visc_cells<<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, nullptr, 0);
+  if (cfg.mode == MCFD_MODE_EXACT) k_visc_cells<true><<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, nullptr, 0);
+  else k_visc_cells<false><<<(C + t - 1) / t, t, 0, s>>>(g, P, vs, w.cell, nullptr, 0);
   k_visc_diffusion<<<(C + t - 1) / t, t, 0, s>>>(g, w.cell, w.diff);
   return cudaGetLastError();
 }
