@@ -1,9 +1,11 @@
-"""Exterior states of pressure inlets, bit for bit: an exact-mode residual of a
-duct whose inlet is a velocity inlet given the states that the full bisections
-give (solver.py:4412-4577 restated in NumPy, the power by the CUDA library's
-pow through PyTorch) equals the residual of the same duct with the real inlet.
-Mach numbers from near stagnation to near sonic, directions from normal to the
-inlet to almost along it.  And the viscosity of Sutherland's law in exact mode
+"""Exterior states of pressure and mass-flow inlets, bit for bit: an exact-mode
+residual of a duct whose inlet is a velocity inlet given the states that the
+full bisections give (solver.py:4412-4577 restated in NumPy, the power by the
+CUDA library's pow through PyTorch) equals the residual of the same duct with
+the real inlet, on every cell.  Pressure inlets: Mach numbers from near
+stagnation to near sonic, directions from normal to the inlet to almost along
+it.  Mass-flow inlets: flow rates from next to none, patches around the
+pairwise sum's leaves and around the 1,024 faces that fit shared memory.  And the viscosity of Sutherland's law in exact mode
 by the same power, read back through the time steps."""
 
 import numpy as np
@@ -111,6 +113,39 @@ def test_pressure_inlet_states_bit_for_bit(cuda_device, ny, vy):
     p = pt * _cuda_pow(t / tt, GAMMA / (GAMMA - 1.0), cuda_device)
     speed = m * np.sqrt(GAMMA * R_GAS * t)
     states = np.column_stack((p / (R_GAS * t), speed * d[0], speed * d[1], p))
+    _check(ny, g, case.numerics, P, faces, states, cuda_device)
+
+
+@pytest.mark.parametrize("ny", (1, 7, 8, 9, 127, 129, 200, 700, 1023, 1024, 1025, 1100))
+@pytest.mark.parametrize("mdot", (1e-6, 0.3, 0.9))
+def test_mass_flow_inlet_states_bit_for_bit(cuda_device, ny, mdot):
+    tt = 1.1 / R_GAS
+    case, g = _duct(ny, ("Mass Flow Inlet", {"mass_flow": mdot, "temperature": tt, "velocity_x": 1.0,
+                                             "velocity_y": -0.1}))
+    (inlet,) = g.mass_flow_inlets
+    faces, d = np.asarray(inlet.faces), np.asarray(inlet.direction, dtype=np.float64)
+    own = np.asarray(g.owners)[faces]
+    normal = np.asarray(g.face_normals).reshape(-1, 2)[faces]
+    proj = -(normal[:, 0] * d[0] + normal[:, 1] * d[1])
+    length = np.asarray(g.face_lengths)[faces]
+    rng = np.random.default_rng(ny)
+    P = np.tile((1.0, 0.3, 0.0, 1.0), (len(g.areas), 1)) + 0.04 * rng.standard_normal((len(g.areas), 4))
+    _, Ph = _residual(g, case.numerics, P, cuda_device)
+    p = Ph[own, 3]
+    cp = GAMMA * R_GAS / (GAMMA - 1.0)
+
+    def below(s):
+        rt = R_GAS * (tt - s * s / (2.0 * cp))
+        return float(np.sum(p / rt * s * proj * length)) < mdot
+
+    low, high = 0.0, np.sqrt(2.0 * cp * tt) * (1.0 - 1e-12)
+    assert not below(high)
+    for _ in range(80):
+        mid = 0.5 * (low + high)
+        low, high = (mid, high) if below(mid) else (low, mid)
+    s = 0.5 * (low + high)
+    rho = p / (R_GAS * (tt - s * s / (2.0 * cp)))
+    states = np.column_stack((rho, np.full(ny, s * d[0]), np.full(ny, s * d[1]), p))
     _check(ny, g, case.numerics, P, faces, states, cuda_device)
 
 
