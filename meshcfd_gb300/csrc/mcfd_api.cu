@@ -377,12 +377,20 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
     set_face(seg_begin[SEG_FAR] + i, d->far_field_faces[i]);
     for (int k = 0; k < 4; ++k) far[4 * i + k] = d->far_field_states[4 * i + k];
   }
-  std::vector<int> bc_ptr(NBP + 1, 0), bc_kind(NBP);
-  std::vector<double> bc_values(4 * NBP), bc_dn(NB);
+  // one face a thread up to kBcMaxParts blocks a patch; a mass-flow inlet, one
+  // speed for all its faces, takes one block
+  std::vector<BcBlock> bc_blocks;
+  std::vector<double> bc_dn(NB);
   for (int64_t k = 0; k < NBP; ++k) {
-    bc_ptr[k + 1] = (int)d->bc_offsets[k + 1];
-    bc_kind[k] = d->bc_kind[k];
-    for (int j = 0; j < 4; ++j) bc_values[4 * k + j] = d->bc_values[4 * k + j];
+    BcBlock b{};
+    b.kind = d->bc_kind[k];
+    b.patch = (int)k;
+    b.first = (int)d->bc_offsets[k];
+    b.last = (int)d->bc_offsets[k + 1];
+    for (int j = 0; j < 4; ++j) b.value[j] = d->bc_values[4 * k + j];
+    const int wanted = (b.last - b.first + kBcThreads - 1) / kBcThreads;
+    b.parts = b.kind == MCFD_BC_MASS_FLOW_INLET ? 1 : std::min(std::max(wanted, 1), kBcMaxParts);
+    for (b.part = 0; b.part < b.parts; ++b.part) bc_blocks.push_back(b);
   }
   for (int64_t i = 0; i < NB; ++i) {
     set_face(seg_begin[SEG_BCX] + i, d->bc_faces[i]);
@@ -673,7 +681,7 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   size_t o_lim_ptr = A.take(bytes_i(C + 1)), o_lim_slot = A.take(bytes_i(NL)),
          o_lim_d = A.take(bytes_d(2 * NL));
   size_t o_par_ptr = A.take(bytes_i(C + 1)), o_par_nb = A.take(bytes_i(NE)), o_par_d = A.take(bytes_d(2 * NE));
-  size_t o_bc_ptr = A.take(bytes_i(NBP + 1)), o_bc_kind = A.take(bytes_i(NBP)), o_bc_values = A.take(bytes_d(4 * NBP)),
+  size_t o_bc_blocks = A.take(bc_blocks.size() * sizeof(BcBlock)),
          o_bc_dn = A.take(bytes_d(NB));
   size_t o_grad_d = A.take(bytes_d(grad_d.size())), o_vb_ptr = A.take(bytes_i(vb_ptr.size())),
          o_vb_j = A.take(bytes_i(ND)), o_diff_owner = A.take(bytes_i(ND)), o_diff_normal = A.take(bytes_d(2 * ND)),
@@ -731,9 +739,7 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   put(o_par_ptr, par_ptr.data(), bytes_i(C + 1));
   put(o_par_nb, par_nb.data(), bytes_i(NE));
   put(o_par_d, par_d.data(), bytes_d(2 * NE));
-  put(o_bc_ptr, bc_ptr.data(), bytes_i(NBP + 1));
-  put(o_bc_kind, bc_kind.data(), bytes_i(NBP));
-  put(o_bc_values, bc_values.data(), bytes_d(4 * NBP));
+  put(o_bc_blocks, bc_blocks.data(), bc_blocks.size() * sizeof(BcBlock));
   put(o_bc_dn, bc_dn.data(), bytes_d(NB));
   put(o_grad_d, grad_d.data(), bytes_d(grad_d.size()));
   put(o_vb_ptr, vb_ptr.data(), bytes_i(vb_ptr.size()));
@@ -823,9 +829,8 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   g.par_rec = AT(const double*, o_par_rec);
   g.par_full = AT(const int*, o_par_full);
   g.n_bc_patches = (int)NBP;
-  g.bc_ptr = AT(const int*, o_bc_ptr);
-  g.bc_kind = AT(const int*, o_bc_kind);
-  g.bc_values = AT(const double*, o_bc_values);
+  g.bc_blocks = AT(const BcBlock*, o_bc_blocks);
+  g.n_bc_blocks = (int)bc_blocks.size();
   g.bc_dn = AT(const double*, o_bc_dn);
   g.bc_ext = AT(double*, o_bc_ext);
   g.bc_ext_dt = AT(double*, o_bc_ext_dt);

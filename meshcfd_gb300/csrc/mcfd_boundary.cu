@@ -1,6 +1,6 @@
 // Exterior states of pressure-inlet, mass-flow-inlet and mass-flow-outlet
-// faces (solver.py:4412-4577): several blocks per boundary patch, one for a
-// mass-flow inlet.
+// faces (solver.py:4412-4577): a block per 128 faces of a boundary patch, one
+// for a mass-flow inlet.
 //
 // * pressure inlet (_pressure_inlet_boundary_states): per face, the Mach
 //   number by 64 bisection steps on the outgoing Riemann invariant, then the
@@ -25,7 +25,7 @@
 namespace mcfd {
 namespace {
 
-constexpr int kBlock = 128;
+constexpr int kBlock = kBcThreads;
 
 __device__ __forceinline__ void flag_patch(DevStatus* st, int bits, int patch) {
   atomicOr(&st->code, bits);
@@ -132,13 +132,11 @@ __device__ __forceinline__ double invariant_at(double m, double dn, double a0, d
 
 template <bool LIBRARY>
 __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* recon, double gamma, double R,
-                               int patch, double* ext) {
+                               const BcBlock& b, double* ext) {
   const int base = g.seg_begin[SEG_BCX];
-  const int j0 = g.bc_ptr[patch], j1 = g.bc_ptr[patch + 1];
-  const double* v = g.bc_values + 4 * (size_t)patch;
-  const double pt = v[0], tt = v[1], dx = v[2], dy = v[3];
+  const double pt = b.value[0], tt = b.value[1], dx = b.value[2], dy = b.value[3];
   const double a0 = sqrt_rn(gamma * R * tt);
-  for (int j = j0 + (int)(blockIdx.y * blockDim.x + threadIdx.x); j < j1; j += (int)(gridDim.y * blockDim.x)) {
+  for (int j = b.first + b.part * kBlock + (int)threadIdx.x; j < b.last; j += b.parts * kBlock) {
     const int f = base + j;
     const St4 q = interior_state(g, P, recon, f);
     const double2 n = g.ff_normal[f];
@@ -192,7 +190,7 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
       const bool finite = isfinite(out.a) && isfinite(out.b) && isfinite(out.c) && isfinite(out.d);
       if (!finite || !(rho > 0.0) || !(p > 0.0)) bits |= MCFD_S_PIN_STATE;
     }
-    if (bits) flag_patch(g.status, bits, patch);
+    if (bits) flag_patch(g.status, bits, b.patch);
     st4(ext + 4 * (size_t)j, out);
   }
 }
@@ -200,7 +198,7 @@ __device__ void pressure_inlet(const DevGeom& g, const double* P, const double* 
 constexpr int kSharedTerms = 1024;  // faces of a mass-flow inlet patch summed in shared memory
 
 __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double* recon, double gamma, double R,
-                                int patch, double* ext) {
+                                const BcBlock& blk, double* ext) {
   __shared__ int s_bad;
   __shared__ int s_below;
   __shared__ int s_leaves;
@@ -208,10 +206,9 @@ __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double*
   __shared__ double s_terms[kSharedTerms], s_weight[kSharedTerms], s_pressure[kSharedTerms], s_sum[kSharedTerms / 64 + 2];
   __shared__ double s_part[kBlock];
   const int base = g.seg_begin[SEG_BCX];
-  const int j0 = g.bc_ptr[patch], j1 = g.bc_ptr[patch + 1], n = j1 - j0;
+  const int patch = blk.patch, j0 = blk.first, j1 = blk.last, n = j1 - j0;
   const bool shared = n <= kSharedTerms;
-  const double* v = g.bc_values + 4 * (size_t)patch;
-  const double mdot = v[0], tt = v[1], dx = v[2], dy = v[3];
+  const double mdot = blk.value[0], tt = blk.value[1], dx = blk.value[2], dy = blk.value[3];
   if (threadIdx.x == 0) {
     s_bad = 0;
     int count = 0;
@@ -315,14 +312,13 @@ __device__ void mass_flow_inlet(const DevGeom& g, const double* P, const double*
   }
 }
 
-__device__ void mass_flow_outlet(const DevGeom& g, const double* P, const double* recon, int patch, double* ext) {
+__device__ void mass_flow_outlet(const DevGeom& g, const double* P, const double* recon, const BcBlock& b, double* ext) {
   const int base = g.seg_begin[SEG_BCX];
-  const int j0 = g.bc_ptr[patch], j1 = g.bc_ptr[patch + 1];
-  const double mdot = g.bc_values[4 * (size_t)patch], total_length = g.bc_values[4 * (size_t)patch + 1];
-  for (int j = j0 + (int)(blockIdx.y * blockDim.x + threadIdx.x); j < j1; j += (int)(gridDim.y * blockDim.x)) {
+  const double mdot = b.value[0], total_length = b.value[1];
+  for (int j = b.first + b.part * kBlock + (int)threadIdx.x; j < b.last; j += b.parts * kBlock) {
     const int f = base + j;
     const St4 q = interior_state(g, P, recon, f);
-    if (q.a <= 0.0 || !isfinite(q.a)) flag_patch(g.status, MCFD_S_MFO_DENSITY, patch);
+    if (q.a <= 0.0 || !isfinite(q.a)) flag_patch(g.status, MCFD_S_MFO_DENSITY, b.patch);
     const double2 n = g.ff_normal[f];
     const double vn = div_rn(mdot, total_length * q.a);
     const double tx = -n.y, ty = n.x;
@@ -335,11 +331,10 @@ template <bool LIBRARY>
 __global__ void __launch_bounds__(kBlock) k_bc_states(DevGeom g, const double* __restrict__ P,
                                                       const double* __restrict__ recon, double gamma, double R,
                                                       double* __restrict__ ext) {
-  const int patch = blockIdx.x;
-  const int kind = g.bc_kind[patch];
-  if (kind == MCFD_BC_PRESSURE_INLET) pressure_inlet<LIBRARY>(g, P, recon, gamma, R, patch, ext);
-  else if (kind == MCFD_BC_MASS_FLOW_OUTLET) mass_flow_outlet(g, P, recon, patch, ext);
-  else if (blockIdx.y == 0) mass_flow_inlet(g, P, recon, gamma, R, patch, ext);
+  const BcBlock b = g.bc_blocks[blockIdx.x];
+  if (b.kind == MCFD_BC_PRESSURE_INLET) pressure_inlet<LIBRARY>(g, P, recon, gamma, R, b, ext);
+  else if (b.kind == MCFD_BC_MASS_FLOW_OUTLET) mass_flow_outlet(g, P, recon, b, ext);
+  else mass_flow_inlet(g, P, recon, gamma, R, b, ext);
 }
 
 }  // namespace
@@ -348,14 +343,10 @@ cudaError_t launch_bc_states(const DevGeom& g, const mcfd_config& cfg, const dou
                              double* ext, cudaStream_t s) {
   if (g.n_bc_patches <= 0) return cudaSuccess;
   count_launch();
-  // enough blocks for one face a thread if one patch held them all
-  const int faces = g.seg_begin[SEG_BCX + 1] - g.seg_begin[SEG_BCX];
-  const int split = (faces + kBlock - 1) / kBlock;
-  const dim3 grid(g.n_bc_patches, split < 1 ? 1 : split > 64 ? 64 : split);
   if (cfg.mode == MCFD_MODE_EXACT)
-    k_bc_states<true><<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
+    k_bc_states<true><<<g.n_bc_blocks, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
   else
-    k_bc_states<false><<<grid, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
+    k_bc_states<false><<<g.n_bc_blocks, kBlock, 0, s>>>(g, P, recon, cfg.gamma, cfg.gas_constant, ext);
   return cudaGetLastError();
 }
 

@@ -15,6 +15,14 @@ namespace mcfd {
 // symmetry planes, velocity inlets, pressure outlets, far field.
 // SEG_BCX: pressure-inlet and mass-flow faces, whose exterior states come from
 // the per-patch boundary kernel (mcfd_boundary.cu) before the flux launch.
+// One block of k_bc_states: its patch, that patch's faces (positions within
+// SEG_BCX) and values, and which of the patch's blocks it is.
+struct BcBlock {
+  int kind, patch, first, last, part, parts;
+  double value[4];
+};
+constexpr int kBcThreads = 128, kBcMaxParts = 64;
+
 enum Segment { SEG_INTERIOR = 0, SEG_PERIODIC, SEG_WALL, SEG_VIN, SEG_POUT, SEG_FAR, SEG_BCX, SEG_COUNT };
 
 // Kinds of dt entries (exterior state used for the boundary spectral radius,
@@ -72,9 +80,8 @@ struct DevGeom {
   const double* ff_far_state;       // [n_far][4]
   // pressure-inlet / mass-flow patches over the SEG_BCX faces
   int n_bc_patches;
-  const int* bc_ptr;       // [patches + 1], positions within SEG_BCX
-  const int* bc_kind;      // [patches]
-  const double* bc_values; // [patches][4]
+  const BcBlock* bc_blocks;  // [n_bc_blocks] (k_bc_states)
+  int n_bc_blocks;
   const double* bc_dn;     // [n_bcx] direction . normal
   double* bc_ext;          // [n_bcx][4] exterior states of the residual (written per evaluation)
   double* bc_ext_dt;       // [n_bcx][4] exterior states of the time step (from cell values)
