@@ -330,32 +330,6 @@ __global__ void __launch_bounds__(kBlock) k_vjp_face(DevGeom g, const double* __
   if (SEG == SEG_FAR && far_bar) st4(far_bar + 4 * (size_t)(f - begin), St4{bar[4], bar[5], bar[6], bar[7]});
 }
 
-// Limiter function of a cell's smallest ratio r >= 0 and its slope there
-// (both 1 and 0 where it is capped): every limiter is nondecreasing in r up to
-// its cap.
-template <int LIMITER>
-__device__ __forceinline__ double limiter_value(double r, double* slope) {
-  *slope = 0.0;
-  if (LIMITER <= 1) {
-    if (!icmp::lt_pos(r, 1.0)) return 1.0;
-    *slope = 1.0;
-    return r;
-  }
-  if (LIMITER == 2) {
-    if (!icmp::gt0(r)) return 0.0;
-    if (!icmp::lt_pos(r, 1.0)) return 1.0;  // 2r / (1 + r) < 1 iff r < 1
-    const double i = div_rn(1.0, 1.0 + r);
-    *slope = 2.0 * i * i;
-    return 2.0 * r * i;
-  }
-  const double eps = 1e-12;
-  const double N = r * r + 2.0 * r + eps, D = r * r + r + 2.0 + eps;
-  if (!icmp::lt_pos(N, D)) return 1.0;
-  const double inv_D = div_rn(1.0, D);
-  *slope = ((2.0 * r + 2.0) * D - N * (2.0 * r + 1.0)) * (inv_D * inv_D);
-  return N * inv_D;
-}
-
 // The cell reverse of one variable: the variable's gradient and extremes,
 // limiter minimum and its first entry, then the reverse of the face states, of
 // the limiter and of the gradient.  One thread takes one variable of a cell
