@@ -218,7 +218,8 @@ inline int seg_threads(int n) {
   return n < 152 * 128 * 16 ? 128 : 256;
 }
 inline int seg_blocks(int n) { return (n + seg_threads(n) - 1) / seg_threads(n); }
-// Faces up to which one launch covers every face segment (k_flux_merged).
+// Faces up to which one launch covers every face segment of the forward
+// fluxes (k_flux_merged).
 // Meshes of more faces launch per segment, where each keeps its own register
 // count (the merged kernel's 76 to 84 against the interior's 64).  RK3 step
 // with one launch against one per segment: 2,970 faces (walls, far field) 130

@@ -177,27 +177,18 @@ __device__ __forceinline__ void flux_tangent_face(const DevGeom& g, const double
   st4(dflux + 4 * (size_t)f, St4{out[0].d[0], out[1].d[0], out[2].d[0], out[3].d[0]});
 }
 
-// One launch per segment, or (up to kMergedFluxFaces faces) all of them in
-// one, the far field's blocks first: its chain of powers is the longest, and
-// as launches of their own the boundary segments ran after the interior one
-// (82 of 604 us of a product on 131,327 cells).
-template <int FLUX, int SEG, bool FO, bool KH>
+// Every segment in one launch, the far field's blocks first: its chain of
+// powers is the longest.  Bound by FP64 issue on large meshes and by that chain
+// on small ones.  A launch per segment was slower at every size, with walls and
+// far field (a product with HLLC fluxes and MUSCL on 208 / 59,080 / 457,080 /
+// 1,230,080 faces 76 / 133 / 581 / 1,443 us, 49 / 94 / 512 / 1,331 us so) and on a
+// periodic box (901,200 faces 1,070 and 1,005 us).
+template <int FLUX, bool FO, bool KH>
 __global__ void __launch_bounds__(kBlock) k_flux_tangent(DevGeom g, const double* __restrict__ P,
                                                          const double* __restrict__ dP,
                                                          const double* __restrict__ recon,
                                                          const double* __restrict__ drecon,
                                                          double* __restrict__ dflux, double gamma) {
-  const int begin = g.seg_begin[SEG];
-  const int f = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (f < g.seg_begin[SEG + 1]) flux_tangent_face<FLUX, SEG, FO, KH>(g, P, dP, recon, drecon, dflux, gamma, f, begin);
-}
-
-template <int FLUX, bool FO, bool KH>
-__global__ void __launch_bounds__(kBlock) k_flux_tangent_merged(DevGeom g, const double* __restrict__ P,
-                                                                const double* __restrict__ dP,
-                                                                const double* __restrict__ recon,
-                                                                const double* __restrict__ drecon,
-                                                                double* __restrict__ dflux, double gamma) {
   int b = blockIdx.x;
 #define MCFD_SEG(SEGV)                                                                                      \
   {                                                                                                         \
@@ -251,30 +242,14 @@ __global__ void __launch_bounds__(kBlock) k_gather_tangent(DevGeom g, const doub
 }
 
 template <int FLUX, bool FO, bool KH>
-void flux_tangent_segments(const DevGeom& g, const double* P, const double* dP, const double* recon,
-                           const double* drecon, double* dflux, double gamma, cudaStream_t s) {
-  const int faces = g.seg_begin[SEG_BCX];
-  if (faces > 0 && faces <= kMergedFluxFaces) {
-    const int t = seg_threads(faces);
-    int blocks = 0;
-    for (int k = 0; k < SEG_BCX; ++k) blocks += (g.seg_begin[k + 1] - g.seg_begin[k] + t - 1) / t;
-    count_launch();
-    k_flux_tangent_merged<FLUX, FO, KH><<<blocks, t, 0, s>>>(g, P, dP, recon, drecon, dflux, gamma);
-    return;
-  }
-#define MCFD_SEG(SEGV)                                                                                     \
-  {                                                                                                        \
-    int n = g.seg_begin[SEGV + 1] - g.seg_begin[SEGV];                                                     \
-    if (n > 0) count_launch(), k_flux_tangent<FLUX, SEGV, FO, KH><<<seg_blocks(n), seg_threads(n), 0, s>>>( \
-                   g, P, dP, recon, drecon, dflux, gamma);                                                 \
-  }
-  MCFD_SEG(SEG_INTERIOR)
-  MCFD_SEG(SEG_PERIODIC)
-  MCFD_SEG(SEG_WALL)
-  MCFD_SEG(SEG_VIN)
-  MCFD_SEG(SEG_POUT)
-  MCFD_SEG(SEG_FAR)
-#undef MCFD_SEG
+void launch_flux_tangent(const DevGeom& g, const double* P, const double* dP, const double* recon,
+                         const double* drecon, double* dflux, double gamma, cudaStream_t s) {
+  const int t = seg_threads(g.seg_begin[SEG_BCX]);
+  int blocks = 0;
+  for (int k = 0; k < SEG_BCX; ++k) blocks += (g.seg_begin[k + 1] - g.seg_begin[k] + t - 1) / t;
+  if (blocks == 0) return;
+  count_launch();
+  k_flux_tangent<FLUX, FO, KH><<<blocks, t, 0, s>>>(g, P, dP, recon, drecon, dflux, gamma);
 }
 
 }  // namespace
@@ -302,17 +277,17 @@ cudaError_t launch_jvp(const DevGeom& g, const mcfd_config& cfg, const double* U
   const bool kh = cfg.reconstruction != MCFD_RECON_MUSCL_PARABOLIC;
   switch (cfg.flux) {
     case MCFD_FLUX_RUSANOV:
-      if (fo) flux_tangent_segments<0, true, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
-      else flux_tangent_segments<0, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      if (fo) launch_flux_tangent<0, true, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      else launch_flux_tangent<0, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
       break;
     case MCFD_FLUX_HLLC:
-      if (fo) flux_tangent_segments<1, true, true>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
-      else if (kh) flux_tangent_segments<1, false, true>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
-      else flux_tangent_segments<1, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      if (fo) launch_flux_tangent<1, true, true>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      else if (kh) launch_flux_tangent<1, false, true>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      else launch_flux_tangent<1, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
       break;
     default:
-      if (fo) flux_tangent_segments<2, true, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
-      else flux_tangent_segments<2, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      if (fo) launch_flux_tangent<2, true, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
+      else launch_flux_tangent<2, false, false>(g, w.P, w.dP, w.recon, w.drecon, w.dflux, cfg.gamma, s);
       break;
   }
   count_launch();
