@@ -794,11 +794,7 @@ int mcfd_geom_create(const mcfd_geom_desc* d, mcfd_geom** out) {
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&h->visc_fork, cudaEventDisableTiming);
   if (err == cudaSuccess) err = cudaEventCreateWithFlags(&h->visc_join, cudaEventDisableTiming);
   if (err != cudaSuccess) {
-    if (h->side.stream) cudaStreamDestroy(h->side.stream);
-    if (h->side.fork) cudaEventDestroy(h->side.fork);
-    if (h->host_status) cudaFreeHost(h->host_status);
-    cudaFree(h->arena);
-    delete h;
+    mcfd_geom_destroy(h);  // whatever of the handle there is
     return MCFD_E_CUDA;
   }
   DevGeom& g = h->g;
