@@ -199,16 +199,16 @@ static cudaError_t stage(mcfd_geom* h, const mcfd_config& cfg, const StageProgra
     if (h->g.n_bc_patches > 0) e = launch_bc_states(h->g, cfg, h->ws.P, nullptr, h->g.bc_ext_dt, s);
     if (e == cudaSuccess) e = cudaEventRecord(h->visc_fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(h->side.stream, h->visc_fork, 0);
-    if (e == cudaSuccess)
-      e = timed(h, MCFD_PROF_OTHER, h->side.stream,
-                [&] { return launch_viscous_residual(h->g, cfg, h->ws.P, h->visc, h->side.stream); });
-    if (e == cudaSuccess) e = cudaEventRecord(h->visc_join, h->side.stream);
-    prog.visc_r = h->visc.r;
     if (e != cudaSuccess) return e;
+    e = timed(h, MCFD_PROF_OTHER, h->side.stream,
+              [&] { return launch_viscous_residual(h->g, cfg, h->ws.P, h->visc, h->side.stream); });
+    const cudaError_t j = cudaEventRecord(h->visc_join, h->side.stream);
+    if (e == cudaSuccess) e = j;
+    prog.visc_r = h->visc.r;
   }
-  if (cfg.reconstruction == MCFD_RECON_MUSCL_LINEAR)
+  if (e == cudaSuccess && cfg.reconstruction == MCFD_RECON_MUSCL_LINEAR)
     e = timed(h, MCFD_PROF_RECONSTRUCT, s, [&] { return MCFD_DISPATCH(cfg, launch_reconstruct(h->g, cfg, h->ws.P, recon_out, s)); });
-  else if (cfg.reconstruction == MCFD_RECON_MUSCL_PARABOLIC)
+  else if (e == cudaSuccess && cfg.reconstruction == MCFD_RECON_MUSCL_PARABOLIC)
     e = timed(h, MCFD_PROF_RECONSTRUCT, s, [&] { return launch_reconstruct_parabolic(h->g, cfg, h->ws.P, recon_out, s); });
   if (e == cudaSuccess && h->g.n_bc_patches > 0) {
     const double* recon = cfg.reconstruction == MCFD_RECON_FIRST_ORDER ? nullptr : recon_out;
