@@ -225,6 +225,15 @@ MCFD_IA_FN double div_rn_recip(double a, double b, u64 X) {
 
 MCFD_IA_FN double div_rn(double a, double b) { return div_rn_recip(a, b, recip_fixed(b)); }
 
+// 1 / b from X = recip_fixed(b) alone, for 2^-1000 < b < 2^1000: X rounded to
+// 53 bits, within 0.51 units in the last place (X is off by a few of its own
+// 64 bits), for a quotient that shares X with a correctly rounded one.
+MCFD_IA_FN double recip_near(double b, u64 X) {
+  const u64 e = bits(b) >> 52;                     // b = 2^(e - 1023) mb / 2^52, 1 / b = 2^(1022 - e) X / 2^63
+  const u64 s = (X >> 11) + ((X >> 10) & 1ull);    // 2^52 .. 2^53
+  return from_bits(((2045ull - e) << 52) + s - kImpl);
+}
+
 // a / b, the same bits as div_rn, in fewer dependent steps, from y =
 // RN(1/b) (div_rn_recip(1.0, b, X)) and X = recip_fixed(b), both of which
 // depend on b alone.  A candidate from one Markstein correction of the
@@ -388,6 +397,7 @@ using ia::div_rn;
 using ia::div_rn_recip;
 using ia::div_rn_fma;
 using ia::recip_fixed;
+using ia::recip_near;
 using ia::mul_rn;
 using ia::negate;
 using ia::plus_zero;
